@@ -308,3 +308,154 @@ def tolerance(case):
     if kind == "gat":
         return {"rel": 3.5e-3, "max": 1.2e-2}    # one TF32 product, fp32 attention: 8e-4, single values 3e-3
     return {"rel": 1e-5}                         # fp32 sums: 2e-8 to 1.5e-6; whole numbers are exact
+
+
+# ------------------------------------------------------------------------------ the same in 64 bits
+class _Product64(torch.autograd.Function):
+    """``A x`` with the transpose at hand for the backward, both sparse, in float64."""
+
+    @staticmethod
+    def forward(ctx, x, a, a_t):
+        ctx.a_t = a_t
+        return a @ x
+
+    @staticmethod
+    def backward(ctx, g):
+        return ctx.a_t @ g.contiguous(), None, None
+
+
+def _sparse64(off, idx, w, n):
+    return torch.sparse_csr_tensor(off, idx, w.double(), (n, n), check_invariants=False)
+
+
+def _gcn64(x, csc, csr, conv1, conv2):
+    n = csc.column_offset.numel() - 1
+    a = _sparse64(csc.column_offset, csc.row_indices, csc.edge_weight, n)
+    a_t = _sparse64(csr.row_offset, csr.column_indices, csr.edge_weight, n)
+    params = [p.detach().double().requires_grad_(True) for p in (conv1.weight, conv1.bias, conv2.weight, conv2.bias)]
+    hidden = torch.relu(_Product64.apply(x.double() @ params[0], a, a_t) + params[1])
+    return _Product64.apply(hidden @ params[2], a, a_t) + params[3], params
+
+
+def _train_step64(x, csc, csr, labels, conv1, conv2, rows=None):
+    logits, params = _gcn64(x, csc, csr, conv1, conv2)
+    if rows is not None:
+        logits = logits[rows]
+    loss = torch.nn.functional.cross_entropy(logits, labels)
+    return {"logits": logits.detach(), "loss": loss.detach(), "grads": list(torch.autograd.grad(loss, params))}
+
+
+def _destinations(off):
+    return torch.repeat_interleave(torch.arange(off.numel() - 1, device=off.device), (off[1:] - off[:-1]).long())
+
+
+def _segment_sum64(v, dst, n):
+    return torch.zeros((n,) + v.shape[1:], dtype=torch.float64, device=v.device).index_add_(0, dst, v)
+
+
+def _segment_softmax64(m, dst, n):
+    top = torch.full((n,), -math.inf, dtype=torch.float64, device=m.device).scatter_reduce_(0, dst, m, "amax")
+    p = torch.exp(m - top[dst])
+    return p / _segment_sum64(p, dst, n)[dst]
+
+
+def _gat64(case, s):
+    """One head at a time; the backward by hand, so that no per-edge rows are kept."""
+    n, heads, dim = case["nodes"], case["heads"], case["dim"]
+    layer, off, idx = s["layer"], s["csc"].column_offset, s["csc"].row_indices
+    x, weight, vec = s["x"].double(), layer.weight.detach().double(), layer.edge_weight.detach().double()[:, 0]
+    h = torch.relu(x @ weight)
+    c = heads * dim
+    dst, src = _destinations(off), idx.long()
+    y, g_h, g_vec = torch.empty_like(h), torch.zeros_like(h), torch.zeros_like(vec)
+    for k in range(heads):
+        cols = slice(k * dim, (k + 1) * dim)
+        hk, a_s, a_d = h[:, cols].contiguous(), vec[cols], vec[c + k * dim:c + (k + 1) * dim]
+        logit = (hk @ a_s)[src] + (hk @ a_d)[dst]
+        alpha = _segment_softmax64(torch.nn.functional.leaky_relu(logit, 0.2), dst, n)
+        y[:, cols] = _sparse64(off, idx, alpha, n) @ hk
+        if not case["backward"]:
+            continue
+        g = s["gy"][:, cols].double()
+        g_alpha = torch.empty_like(alpha)
+        step = 1 << 22
+        for e in range(0, alpha.numel(), step):
+            g_alpha[e:e + step] = (g[dst[e:e + step]] * hk[src[e:e + step]]).sum(1)
+            g_h[:, cols].index_add_(0, src[e:e + step], alpha[e:e + step, None] * g[dst[e:e + step]])
+        g_logit = alpha * (g_alpha - _segment_sum64(alpha * g_alpha, dst, n)[dst])
+        g_logit = torch.where(logit > 0, g_logit, 0.2 * g_logit)
+        by_src, by_dst = _segment_sum64(g_logit, src, n), _segment_sum64(g_logit, dst, n)
+        g_h[:, cols] += by_src[:, None] * a_s + by_dst[:, None] * a_d
+        g_vec[cols], g_vec[c + k * dim:c + (k + 1) * dim] = by_src @ hk, by_dst @ hk
+    if not case["backward"]:
+        return y
+    return y, [x.t() @ (g_h * (h > 0)), g_vec[:, None]]
+
+
+def _edge_ops64(case, s):
+    n = case["nodes"]
+    dst, src = _destinations(s["csc"].column_offset), s["csc"].row_indices.long()
+    alpha, g_score = [], []
+    for k in range(case["heads"]):
+        a, g = _segment_softmax64(s["score"].detach()[:, k].double(), dst, n), s["g_score"][:, k].double()
+        alpha.append(a)
+        g_score.append(a * (g - _segment_sum64(a * g, dst, n)[dst]))
+    return {"alpha": torch.stack(alpha, 1), "g_score": torch.stack(g_score, 1), "edge": s["x"].detach().double()[src],
+            "g_x": _segment_sum64(s["g_edge"].double(), src, n), "node": _segment_sum64(s["msg"].detach().double(), dst, n),
+            "g_msg": s["g_node"].double()[dst]}
+
+
+def _convert64(case, s):
+    """The weights; the whole numbers beside them are compared as they are."""
+    n = case["nodes"]
+    src, dst = s["ei"]
+    w = torch.ones(src.numel(), device="cuda") if s["w"] is None else s["w"]
+    loop_w = torch.ones(n, device="cuda")
+    loops = torch.nonzero(src == dst)[:, 0]                       # a node's last loop entry gives its weight
+    at = torch.full((n,), -1, device="cuda").scatter_reduce_(0, src[loops].long(), loops, "amax")
+    loop_w = torch.where(at >= 0, w[at.clamp(min=0)], loop_w)
+    ids = torch.arange(n, dtype=torch.int32, device="cuda")
+    keep = src != dst
+    src, dst, w = torch.cat([src[keep], ids]), torch.cat([dst[keep], ids]), torch.cat([w[keep], loop_w]).double()
+    inv = torch.zeros(n, dtype=torch.float64, device="cuda").index_add_(0, dst, w).rsqrt()
+    w = inv[src] * w * inv[dst]
+    return [None, None, w[torch.sort(dst, stable=True)[1]], None, None, w[torch.sort(src, stable=True)[1]]]
+
+
+def exact(case, seed):
+    """What ``run`` returns, from plain torch in float64 on the structure that the inputs hold.  A sampled
+    batch is whole numbers: the exact values are those of the step on that batch."""
+    s = prepare(case, seed)
+    kind = case["kind"]
+    if kind == "gcn_step":
+        return _train_step64(s["x"], s["csc"], s["csr"], s["labels"], s["conv1"], s["conv2"])
+    if kind == "gcn_infer":
+        with torch.no_grad():
+            return _gcn64(s["x"], s["csc"], s["csr"], s["conv1"], s["conv2"])[0]
+    if kind == "minibatch":
+        b = sampling.sample_one([case["fan0"], case["fan1"]], s["csc"].column_offset, s["csc"].row_indices, s["seeds"], seed=s["seed"])
+        nodes = b.local2global.long()
+        rows = torch.searchsorted(b.local2global, s["seeds"])
+        return _train_step64(s["x"][nodes], b.csc, b.csr, s["labels"][nodes][rows], s["conv1"], s["conv2"], rows)
+    if kind in ("spmm", "appnp"):
+        n, x = case["nodes"], s["x"].detach().double()
+        a = _sparse64(s["csc"].column_offset, s["csc"].row_indices, s["csc"].edge_weight, n)
+        if kind == "spmm" and not case["backward"]:
+            return a @ x
+        a_t = _sparse64(s["csr"].row_offset, s["csr"].column_indices, s["csr"].edge_weight, n)
+        g = s["gy"].double()
+        if kind == "spmm":
+            return a @ x, a_t @ g
+        y, gx = x, torch.zeros_like(g)
+        for _ in range(case["hops"]):
+            y = 0.1 * x + 0.9 * (a @ y)
+            gx = gx + 0.1 * g
+            g = 0.9 * (a_t @ g)
+        return y, gx + g
+    if kind == "gat":
+        with torch.no_grad():
+            return _gat64(case, s)
+    if kind == "edge_ops":
+        with torch.no_grad():
+            return _edge_ops64(case, s)
+    return _convert64(case, s)
