@@ -223,6 +223,24 @@ def test_gat_layer_fused_and_unfused_agree(cuda):
         assert (a - b).abs().max().item() <= 2e-4 * (b.abs().max().item() + 1e-30)
 
 
+@pytest.mark.parametrize("edges", [1, 3, 5, 4099])
+@pytest.mark.parametrize("c", [1, 2, 3, 4, 6, 30, 64, 126, 132, 260])
+def test_scatter_to_edge_backward_by_source(cuda, c, edges):
+    """Vector reductions of 4, 2 and 1 values, edge counts that end inside a group of edges.  A sum of k terms in
+    any order is off by at most (k - 1) * 2^-24 of the sum of magnitudes."""
+    n, rng = 37, np.random.default_rng(c + edges)
+    idx, off = random_csc(rng, n, edges)
+    csc = cuda.CSC(dev(idx), dev(off), None)
+    m = rng.standard_normal((edges, c)).astype(np.float32)
+    x = dev(np.zeros((n, c), np.float32)).requires_grad_(True)
+    cuda.ScatterToEdge(x, csc, "src").backward(dev(m))
+    want, mag = np.zeros((n, c)), np.zeros((n, c))
+    np.add.at(want, idx, m.astype(np.float64))
+    np.add.at(mag, idx, np.abs(m).astype(np.float64))
+    terms = max(int(np.bincount(idx, minlength=n).max()), 1)
+    assert np.all(np.abs(host(x.grad) - want) <= terms * 2.0**-24 * mag)
+
+
 def attention_truth(h, a_src, a_dst, idx, off, slope=0.2):
     """Differentiable float64 restatement of the edge phase with plain tensor operations."""
     n, heads, dim = h.shape[0], a_src.shape[0], a_src.shape[1]
