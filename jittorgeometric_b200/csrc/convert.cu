@@ -16,17 +16,27 @@
 // removal and the appended loops are folded into it: removed entries are simply never counted),
 // the last pass writes the caller's output arrays.  Offsets are found from the sorted keys by
 // boundary detection; nothing uses floating-point atomics, so results are run-to-run identical.
-// HBM-bound: about 28 bytes per entry and pass (4 histogram read, 12 read, 12 write).
+// About 20 bytes per entry and pass (4 histogram read, 8 read, 8 write; 12 more with weights to carry).  The scatter
+// is bound by the SM, not by DRAM: 37 shared-memory and load/store wavefronts and some 60 integer instructions per
+// 32 entries (ranks, staging, write-out) are 1.65 ms of a 285 M-entry pass against 0.7 ms for its bytes.
 #include "common.cuh"
 #include "scan.cuh"
 
 namespace jg {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 8;
-constexpr int kSortTile = kSortThreads * kSortItems;  // 2048 entries per tile
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kRadix = 256;
+// Entries per thread of a tile.  Sixteen halve the count matrix and its scans and lengthen the write runs (285 M
+// unit-weight entries, three passes, two formats: 14.9 against 15.9 ms), but a third array to carry spills
+// (30 M weighted entries: 3.1 against 2.6 ms), and a list of fewer than some 2 M entries would leave SMs
+// without a tile.
+constexpr int kItemsFew = 8, kItemsMany = 16;
+constexpr int64_t kManyEntries = (int64_t)1 << 21;
+static inline int sort_items(int64_t count, bool carry_w) { return !carry_w && count >= kManyEntries ? kItemsMany : kItemsFew; }
+static inline int64_t sort_tiles(int64_t count, int items) {
+    return (count + (int64_t)kSortThreads * items - 1) / ((int64_t)kSortThreads * items);
+}
 
 // ------------------------------------------------------------------------------- digit-major scan
 // The per-tile digit counts live as matrix[tile][digit] (rows of 256 counts, written and read
@@ -45,7 +55,9 @@ __global__ void __launch_bounds__(kRadix) colscan_chunk_sums(const int* __restri
     chunk_sums[(int64_t)blockIdx.x * kRadix + threadIdx.x] = sum;
 }
 
-__global__ void __launch_bounds__(kRadix) colscan_chunks(int* __restrict__ chunk_sums, int64_t n_chunks) {
+// `total` (or null) receives the number of entries counted.
+__global__ void __launch_bounds__(kRadix) colscan_chunks(int* __restrict__ chunk_sums, int64_t n_chunks,
+                                                         unsigned long long* __restrict__ total) {
     __shared__ int s_warp[32];
     __shared__ int s_total;
     int run = 0;
@@ -55,6 +67,7 @@ __global__ void __launch_bounds__(kRadix) colscan_chunks(int* __restrict__ chunk
         run += v;
     }
     const int base = block_exclusive_scan(run, &s_total, s_warp);   // entries with a smaller digit
+    if (total && threadIdx.x == 0) *total = (unsigned long long)s_total;
     for (int64_t c = 0; c < n_chunks; c++) chunk_sums[c * kRadix + threadIdx.x] += base;
 }
 
@@ -67,6 +80,27 @@ __global__ void __launch_bounds__(kRadix) colscan_apply(int* __restrict__ matrix
         const int v = matrix[t * kRadix + threadIdx.x];
         matrix[t * kRadix + threadIdx.x] = run;
         run += v;
+    }
+}
+
+// The same in one launch for a matrix of at most kChunkTiles rows.
+__global__ void __launch_bounds__(kRadix) colscan_small(int* __restrict__ matrix, int n_tiles, unsigned long long* __restrict__ total) {
+    __shared__ int s_warp[32];
+    __shared__ int s_total;
+    int sum = 0;
+#pragma unroll 16
+    for (int t = 0; t < n_tiles; t++) sum += matrix[t * kRadix + threadIdx.x];
+    int run = block_exclusive_scan(sum, &s_total, s_warp);
+    if (total && threadIdx.x == 0) *total = (unsigned long long)s_total;
+    for (int t0 = 0; t0 < n_tiles; t0 += 16) {
+        int v[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) v[i] = t0 + i < n_tiles ? matrix[(t0 + i) * kRadix + threadIdx.x] : 0;
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            if (t0 + i < n_tiles) matrix[(t0 + i) * kRadix + threadIdx.x] = run;
+            run += v[i];
+        }
     }
 }
 
@@ -158,40 +192,88 @@ __device__ __forceinline__ int digit_of(const Elem& e, int shift, int from_idx) 
 
 // SORTED: the source is a sorted buffer (mode 0); a separate instantiation, so that the register needs of the
 // first pass's element loader do not lower the occupancy of the other passes.
-template <bool SORTED>
-__global__ void __launch_bounds__(kSortThreads) sort_hist_kernel(SortSrc s, int shift, int from_idx, int* __restrict__ matrix,
-                                                                 int64_t n_tiles) {
+constexpr int kHistThreads = kSortThreads;
+template <bool SORTED, int ITEMS>
+__global__ void __launch_bounds__(kHistThreads) sort_hist_kernel(SortSrc s, int shift, int from_idx, int* __restrict__ matrix) {
     __shared__ int s_hist[kRadix];
+    constexpr int kSortTile = kSortThreads * ITEMS;
+    constexpr int kRounds = ITEMS;
+    constexpr int kBatch = 8;
+    static_assert(kRounds % kBatch == 0, "a tile is read in whole batches");
     s_hist[threadIdx.x] = 0;
     __syncthreads();
     const int64_t base = (int64_t)blockIdx.x * kSortTile;
+    const int64_t count = list_count(s);
     if (SORTED) {
         // sorted-buffer passes: only the array the digit comes from is read (half the bytes of a full element)
         const int32_t* from = from_idx ? s.idx : s.key;
-        const int64_t count = s.dcount ? (int64_t)*s.dcount : s.count;
-        int32_t v[kSortItems];
+        if (base + kSortTile <= count && reinterpret_cast<uintptr_t>(from) % 16 == 0) {
+            int4 v[kRounds / 4];
 #pragma unroll
-        for (int i = 0; i < kSortItems; i++) {
-            const int64_t p = base + (int64_t)i * kSortThreads + threadIdx.x;
-            v[i] = p < count ? from[p] : -1;
+            for (int i = 0; i < kRounds / 4; i++) v[i] = reinterpret_cast<const int4*>(from + base)[i * kHistThreads + threadIdx.x];
+#pragma unroll
+            for (int i = 0; i < kRounds / 4; i++) {
+                atomicAdd(&s_hist[(v[i].x >> shift) & (kRadix - 1)], 1);
+                atomicAdd(&s_hist[(v[i].y >> shift) & (kRadix - 1)], 1);
+                atomicAdd(&s_hist[(v[i].z >> shift) & (kRadix - 1)], 1);
+                atomicAdd(&s_hist[(v[i].w >> shift) & (kRadix - 1)], 1);
+            }
+        } else {
+            for (int i = 0; i < kRounds; i++) {
+                const int64_t p = base + (int64_t)i * kHistThreads + threadIdx.x;
+                if (p < count) atomicAdd(&s_hist[(from[p] >> shift) & (kRadix - 1)], 1);
+            }
         }
-#pragma unroll
-        for (int i = 0; i < kSortItems; i++)
-            if (v[i] >= 0) atomicAdd(&s_hist[(v[i] >> shift) & (kRadix - 1)], 1);
     } else {
-        const int64_t count = list_count(s);
-        Raw raw[kSortItems];
+#pragma unroll 1
+        for (int i0 = 0; i0 < kRounds; i0 += kBatch) {
+            Raw raw[kBatch];
 #pragma unroll
-        for (int i = 0; i < kSortItems; i++) raw[i] = load_raw(s, base + (int64_t)i * kSortThreads + threadIdx.x, count);   // all loads in flight
+            for (int i = 0; i < kBatch; i++) raw[i] = load_raw(s, base + (int64_t)(i0 + i) * kHistThreads + threadIdx.x, count);   // all loads in flight
 #pragma unroll
-        for (int i = 0; i < kSortItems; i++) {
-            const Elem e = finish_elem(s, base + (int64_t)i * kSortThreads + threadIdx.x, count, raw[i]);
-            if (e.valid) atomicAdd(&s_hist[digit_of(e, shift, from_idx)], 1);
+            for (int i = 0; i < kBatch; i++) {
+                const Elem e = finish_elem(s, base + (int64_t)(i0 + i) * kHistThreads + threadIdx.x, count, raw[i]);
+                if (e.valid) atomicAdd(&s_hist[digit_of(e, shift, from_idx)], 1);
+            }
         }
     }
     __syncthreads();
     matrix[(int64_t)blockIdx.x * kRadix + threadIdx.x] = s_hist[threadIdx.x];   // [tile][digit]: one coalesced row
-    (void)n_tiles;
+}
+
+// First-pass counts of BOTH formats from one read of the COO list (mode 1): by destination and by source.
+template <int ITEMS>
+__global__ void __launch_bounds__(kHistThreads) sort_hist_both_kernel(SortSrc s, int* __restrict__ by_dst, int* __restrict__ by_src) {
+    __shared__ int s_hist[2][kRadix];
+    constexpr int kSortTile = kSortThreads * ITEMS;
+    constexpr int kRounds = ITEMS;
+    constexpr int kBatch = 8;
+    static_assert(kRounds % kBatch == 0, "a tile is read in whole batches");
+    s_hist[0][threadIdx.x] = 0;
+    s_hist[1][threadIdx.x] = 0;
+    __syncthreads();
+    const int64_t base = (int64_t)blockIdx.x * kSortTile;
+    const int64_t count = list_count(s);
+    s.coo_w = nullptr;
+    s.loop_w = nullptr;
+#pragma unroll 1
+    for (int i0 = 0; i0 < kRounds; i0 += kBatch) {
+        Raw raw[kBatch];
+#pragma unroll
+        for (int i = 0; i < kBatch; i++) raw[i] = load_raw(s, base + (int64_t)(i0 + i) * kHistThreads + threadIdx.x, count);
+#pragma unroll
+        for (int i = 0; i < kBatch; i++) {
+            const Elem e = finish_elem(s, base + (int64_t)(i0 + i) * kHistThreads + threadIdx.x, count, raw[i]);
+            if (e.valid) {
+                const int src = s.by == 0 ? e.key : e.idx, dst = s.by == 0 ? e.idx : e.key;
+                atomicAdd(&s_hist[0][dst & (kRadix - 1)], 1);
+                atomicAdd(&s_hist[1][src & (kRadix - 1)], 1);
+            }
+        }
+    }
+    __syncthreads();
+    by_dst[(int64_t)blockIdx.x * kRadix + threadIdx.x] = s_hist[0][threadIdx.x];
+    by_src[(int64_t)blockIdx.x * kRadix + threadIdx.x] = s_hist[1][threadIdx.x];
 }
 
 struct SortDst {
@@ -204,49 +286,85 @@ struct SortDst {
 // order of the source list because warp w reads one contiguous range of 32 * kSortItems entries.
 // HAS_W = false: every weight is 1 (no input weights), so the sort moves (key, index) pairs only and
 // the caller writes the weights afterwards; a third less traffic per pass.
-template <bool HAS_W>
-__global__ void __launch_bounds__(kSortThreads, 4) sort_scatter_kernel(SortSrc s, SortDst d, int shift, int from_idx,
-                                                                    const int* __restrict__ matrix, int64_t n_tiles) {
+// SORTED: the source is a buffer (mode 0); the first pass's element loader is an instantiation of its own.
+template <bool HAS_W, bool SORTED, int ITEMS>
+__global__ void __launch_bounds__(kSortThreads, ITEMS == kItemsMany ? 3 : 4) sort_scatter_kernel(SortSrc s, SortDst d, int shift, int from_idx,
+                                                                                                const int* __restrict__ matrix) {
+    constexpr int kSortItems = ITEMS;
+    constexpr int kSortTile = kSortThreads * ITEMS;
     extern __shared__ __align__(16) unsigned char smem[];
-    int* s_whist = reinterpret_cast<int*>(smem);                       // [kSortWarps][kRadix]
+    int2* s_pair = reinterpret_cast<int2*>(smem);                      // [kSortTile] (key, index): one 8-byte access per element
+    int* s_whist = reinterpret_cast<int*>(s_pair + kSortTile);         // [kSortWarps][kRadix]
     int* s_gbase = s_whist + kSortWarps * kRadix;                      // [kRadix] global offset of a digit for this tile
     int* s_scan = s_gbase + kRadix;                                    // [32]
-    int2* s_pair = reinterpret_cast<int2*>(s_scan + 32);               // [kSortTile] (key, index): one 8-byte access per element
-    float* s_w = reinterpret_cast<float*>(s_pair + kSortTile);         // [kSortTile]
+    float* s_w = reinterpret_cast<float*>(s_scan + 32);                // [kSortTile], HAS_W only
     __shared__ int s_total;
 
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int tile_first = matrix[(int64_t)blockIdx.x * kRadix + threadIdx.x];   // this tile's global start of digit `threadIdx.x`: fetched first, needed last
-    for (int i = threadIdx.x; i < kSortWarps * kRadix; i += kSortThreads) s_whist[i] = 0;
-    __syncthreads();
-
+    const int64_t count = list_count(s);
     const int64_t wbase = (int64_t)blockIdx.x * kSortTile + (int64_t)wid * (32 * kSortItems);
-    Elem el[kSortItems];
-    int dig[kSortItems];
-    int rank[kSortItems];
-    int* my_hist = s_whist + wid * kRadix;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    // every load of the tile first (independent, all in flight), the ranking rounds after them: with the load
-    // inside the round each of the eight rounds waited for its own memory latency behind the warp barriers
-    {
-        const int64_t count = list_count(s);
+    static_assert(kSortThreads == kRadix, "one thread per digit");
+    const int tile_first = matrix[(int64_t)blockIdx.x * kRadix + threadIdx.x];   // this tile's global start of digit `threadIdx.x`: fetched first, needed last
+    int32_t key[kSortItems], idx[kSortItems];
+    float wt[HAS_W ? kSortItems : 1];
+    unsigned valid = 0;
+    // every load of the tile first (independent, all in flight), the ranking rounds after them
+    if (SORTED) {
+#pragma unroll
+        for (int r = 0; r < kSortItems; r++) {
+            const int64_t p = wbase + r * 32 + lane;
+            const bool in = p < count;
+            key[r] = in ? s.key[p] : 0;
+            idx[r] = in ? s.idx[p] : 0;
+            if (HAS_W) wt[r] = in ? s.w[p] : 0.f;
+            valid |= in ? 1u << r : 0u;
+        }
+    } else {
         Raw raw[kSortItems];
 #pragma unroll
         for (int r = 0; r < kSortItems; r++) raw[r] = load_raw(s, wbase + r * 32 + lane, count);
 #pragma unroll
-        for (int r = 0; r < kSortItems; r++) el[r] = finish_elem(s, wbase + r * 32 + lane, count, raw[r]);
+        for (int r = 0; r < kSortItems; r++) {
+            const Elem e = finish_elem(s, wbase + r * 32 + lane, count, raw[r]);
+            key[r] = e.key; idx[r] = e.idx;
+            if (HAS_W) wt[r] = e.w;
+            valid |= e.valid ? 1u << r : 0u;
+        }
     }
+    int* my_hist = s_whist + wid * kRadix;
+#pragma unroll
+    for (int i = 0; i < kRadix / 32; i++) my_hist[i * 32 + lane] = 0;
+    __syncwarp();
+    const unsigned lt_mask = (1u << lane) - 1u;
+    // Ranking: lanes with the same digit find each other by a match mask, the first of them takes the group's
+    // places with ONE shared-memory atomic and hands the start round.  The rounds' atomics are issued one behind
+    // the other and their results picked up afterwards, so a round does not wait for the one before it (a
+    // read, a warp barrier, a write and another warp barrier per round were a chain of eight shared-memory
+    // latencies: 2.05 ms per pass of 285 M pairs).
+    // place of an element: start of its group (valid in the group's first lane until it is handed round) in the low
+    // 16 bits, that lane's number and the elements before this one in the bytes above - one register per element
+    static_assert(kSortTile <= 1 << 16, "tile slots are kept in 16 bits");
+    unsigned place[kSortItems];
 #pragma unroll
     for (int r = 0; r < kSortItems; r++) {
-        dig[r] = el[r].valid ? digit_of(el[r], shift, from_idx) : kRadix;  // kRadix: not an element
-        const unsigned peers = __match_any_sync(kFull, dig[r]);
-        int before = 0;
-        if (el[r].valid) before = my_hist[dig[r]];
-        __syncwarp();
-        rank[r] = before + __popc(peers & lt_mask);
-        if (el[r].valid && (peers & lt_mask) == 0) my_hist[dig[r]] = before + __popc(peers);
+        const bool ok = (valid >> r) & 1u;
+        const unsigned dg = ((unsigned)(from_idx ? idx[r] : key[r]) >> shift) & (kRadix - 1);
+        // lanes with this lane's digit, one vote per digit bit.  __match_any_sync gives the same mask, but it
+        // takes one step per distinct value among the lanes (25 of 32 on shuffled edges) on a pipe that was
+        // 82 % busy with it and set the pace of the whole pass.
+        unsigned peers = __ballot_sync(kFull, ok);
+#pragma unroll
+        for (int b = 0; b < 8; b++) {
+            const unsigned bit = (dg >> b) & 1u;
+            peers &= __ballot_sync(kFull, bit) ^ (bit - 1u);
+        }
+        place[r] = (unsigned)(__ffs(peers) - 1) << 16 | (unsigned)__popc(peers & lt_mask) << 24;
+        if (ok && (peers & lt_mask) == 0) place[r] += (unsigned)atomicAdd(&my_hist[dg], __popc(peers));
         __syncwarp();
     }
+#pragma unroll
+    for (int r = 0; r < kSortItems; r++)
+        place[r] = (__shfl_sync(kFull, place[r], (place[r] >> 16) & 31u) & 0xffffu) + (place[r] >> 24);
     __syncthreads();
     // one thread per digit: exclusive prefix over warps, tile total
     {
@@ -260,27 +378,27 @@ __global__ void __launch_bounds__(kSortThreads, 4) sort_scatter_kernel(SortSrc s
             cnt_w[w] = s_whist[w * kRadix + dgt];
             run += cnt_w[w];
         }
-        const int start = block_exclusive_scan(run, &s_total, s_scan);
-        int at = start;
+        const int first = block_exclusive_scan(run, &s_total, s_scan);
+        int at = first;
 #pragma unroll
         for (int w = 0; w < kSortWarps; w++) {
             s_whist[w * kRadix + dgt] = at;
             at += cnt_w[w];
         }
-        s_gbase[dgt] = tile_first - start;  // global position = gbase + tile slot
-        (void)n_tiles;
+        s_gbase[dgt] = tile_first - first;  // global position = gbase + tile slot
     }
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < kSortItems; r++) {
-        if (el[r].valid) {
-            const int q = my_hist[dig[r]] + rank[r];
-            s_pair[q] = make_int2(el[r].key, el[r].idx);
-            if (HAS_W) s_w[q] = el[r].w;
+        if ((valid >> r) & 1u) {
+            const int q = my_hist[((from_idx ? idx[r] : key[r]) >> shift) & (kRadix - 1)] + (int)place[r];
+            s_pair[q] = make_int2(key[r], idx[r]);
+            if (HAS_W) s_w[q] = wt[r];
         }
     }
     __syncthreads();
     const int total = s_total;
+#pragma unroll 4
     for (int q = threadIdx.x; q < total; q += kSortThreads) {
         const int2 e = s_pair[q];
         const int64_t g = (int64_t)s_gbase[((from_idx ? e.y : e.x) >> shift) & (kRadix - 1)] + q;   // the digit again, from the element
@@ -290,47 +408,76 @@ __global__ void __launch_bounds__(kSortThreads, 4) sort_scatter_kernel(SortSrc s
     }
 }
 
-constexpr size_t kScatterSmem = sizeof(int) * (kSortWarps * kRadix + kRadix + 32) +
-                                sizeof(int2) * kSortTile + sizeof(float) * kSortTile;
+constexpr size_t scatter_smem(bool has_w, int items) {
+    return (size_t)kSortThreads * items * (has_w ? 12 : 8) + sizeof(int) * (kSortWarps * kRadix + kRadix + 32);
+}
+
+typedef void (*ScatterFn)(SortSrc, SortDst, int, int, const int*);
+static ScatterFn scatter_fn(bool has_w, bool sorted, int items) {
+    if (has_w) return sorted ? sort_scatter_kernel<true, true, kItemsFew> : sort_scatter_kernel<true, false, kItemsFew>;
+    if (items == kItemsFew) return sorted ? sort_scatter_kernel<false, true, kItemsFew> : sort_scatter_kernel<false, false, kItemsFew>;
+    return sorted ? sort_scatter_kernel<false, true, kItemsMany> : sort_scatter_kernel<false, false, kItemsMany>;
+}
+
+static void launch_hist(const SortSrc& src, int shift, int from_idx, int* matrix, int64_t tiles, int items, cudaStream_t st) {
+    const bool sorted = src.mode == 0;
+    auto kern = items == kItemsFew ? (sorted ? sort_hist_kernel<true, kItemsFew> : sort_hist_kernel<false, kItemsFew>)
+                                   : (sorted ? sort_hist_kernel<true, kItemsMany> : sort_hist_kernel<false, kItemsMany>);
+    kern<<<(unsigned)tiles, kHistThreads, 0, st>>>(src, shift, from_idx, matrix);
+}
 
 // ------------------------------------------------------------------------------- small kernels
 // off[k] = first position whose key is >= k, for k in [0, n]; keys sorted, E entries.
-__global__ void offsets_from_sorted_keys(const int32_t* __restrict__ key, int64_t E_host,
-                                         const unsigned long long* __restrict__ dcount, int64_t n, int32_t* __restrict__ off) {
-    // four positions per thread: one 16-byte load of their keys (when aligned) and the key before them
+// Each thread takes four groups of four consecutive positions, a block's width apart, and issues all their loads
+// before it looks at one (285 M keys: 0.39 -> 0.38 ms; the runs of empty rows, written one by one, are the rest).
+constexpr int kOffThreads = 256;
+constexpr int kOffGroups = 4;
+constexpr int64_t kOffTile = (int64_t)kOffThreads * kOffGroups * 4;
+__global__ void __launch_bounds__(kOffThreads) offsets_from_sorted_keys(const int32_t* __restrict__ key, int64_t E_host,
+                                                                        const unsigned long long* __restrict__ dcount, int64_t n,
+                                                                        int32_t* __restrict__ off) {
     const int64_t E = dcount ? (int64_t)*dcount : E_host;
-    const int64_t j0 = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-    if (j0 > E) return;
-    int64_t prev = j0 == 0 ? -1 : key[j0 - 1];
-    int32_t k4[4];
-    if (j0 + 4 <= E && reinterpret_cast<uintptr_t>(key) % 16 == 0) {
-        const int4 v = *reinterpret_cast<const int4*>(key + j0);
-        k4[0] = v.x; k4[1] = v.y; k4[2] = v.z; k4[3] = v.w;
-    } else {
+    const int64_t base = (int64_t)blockIdx.x * kOffTile + 4 * threadIdx.x;
+    const bool vec = reinterpret_cast<uintptr_t>(key) % 16 == 0;
+    int4 k4[kOffGroups];
+    int32_t before[kOffGroups];
 #pragma unroll
-        for (int i = 0; i < 4; i++) k4[i] = j0 + i < E ? key[j0 + i] : 0;
+    for (int g = 0; g < kOffGroups; g++) {
+        const int64_t j = base + (int64_t)g * kOffThreads * 4;
+        before[g] = j > 0 && j <= E ? __ldg(key + j - 1) : -1;
+        k4[g] = make_int4(0, 0, 0, 0);
+        if (vec && j + 4 <= E) {
+            k4[g] = __ldg(reinterpret_cast<const int4*>(key + j));
+        } else {
+            if (j < E) k4[g].x = __ldg(key + j);
+            if (j + 1 < E) k4[g].y = __ldg(key + j + 1);
+            if (j + 2 < E) k4[g].z = __ldg(key + j + 2);
+            if (j + 3 < E) k4[g].w = __ldg(key + j + 3);
+        }
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int64_t j = j0 + i;
-        if (j > E) break;
-        const int64_t hi = j == E ? n : k4[i];
-        for (int64_t k = prev + 1; k <= hi; k++) off[k] = (int32_t)j;
-        prev = hi;
+    for (int g = 0; g < kOffGroups; g++) {
+        const int64_t j0 = base + (int64_t)g * kOffThreads * 4;
+        int64_t prev = before[g];
+        const int32_t k[4] = {k4[g].x, k4[g].y, k4[g].z, k4[g].w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int64_t j = j0 + i;
+            if (j > E) break;
+            const int64_t hi = j == E ? n : k[i];
+            for (int64_t v = prev + 1; v <= hi; v++) off[v] = (int32_t)j;
+            prev = hi;
+        }
     }
 }
+static inline unsigned offset_blocks(int64_t count) { return (unsigned)(count / kOffTile + 1); }   // positions 0 .. count
 
 __global__ void set_count_kernel(unsigned long long* p, unsigned long long v) { *p = v; }
 
-// Valid-entry count of the first pass (input entries that are not (v,v), plus loops).
-__global__ void count_kept_kernel(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64_t e0,
-                                  unsigned long long* __restrict__ kept) {
-    unsigned long long c = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < e0; i += (int64_t)gridDim.x * blockDim.x)
-        c += src[i] != dst[i];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(kept, c);
+static int launch_set_count(unsigned long long* p, unsigned long long v, cudaStream_t st) {
+    set_count_kernel<<<1, 1, 0, st>>>(p, v);
+    JG_LAUNCH_CHECK();
+    return JG_OK;
 }
 
 // Weight of the loop appended for node v: the fill value, or the weight of the LAST (v,v) input
@@ -346,11 +493,23 @@ __global__ void loop_weight_kernel(const int* __restrict__ last, const float* __
     if (v < n) loop_w[v] = last[v] >= 0 ? (w ? w[last[v]] : 1.f) : fill;
 }
 
-// deg[v] = sum of the raw weights of column v in list order (sequential fp32 adds, the order a
-// host scatter-add takes); dis = deg^-1/2 correctly rounded through double.
-__global__ void degree_kernel(const int32_t* __restrict__ off, const float* __restrict__ w, int64_t n, int unit,
-                              float* __restrict__ dis) {
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// deg[v] = sum of the raw weights of column v; dis = deg^-1/2 correctly rounded through double.  Columns of up to
+// kLongColumn entries are added sequentially in list order, the order a host scatter-add takes: by one thread up to
+// kThreadColumn entries, else by a warp that reads 32 entries at a time and adds them one by one.  A longer column
+// is added by a block - every thread a strided part, then a fixed tree - which is closer to the exact sum than the
+// sequential order.  With one thread per column whatever its length, a 30 M-edge weighted R-MAT list spent 1.86 of
+// the conversion's 4.5 ms here, behind the threads that own the hubs.
+// Columns beyond one thread's share are listed: warp columns from the front of `list`, block columns from its back,
+// count[0] and count[1] of them (zeroed by the launcher), so that neighbouring hubs spread over the device.
+constexpr int kThreadColumn = 64;
+constexpr int kLongColumn = 4096;
+constexpr int kDegThreads = 256;
+__device__ __forceinline__ float inv_sqrt_degree(float deg) { return (float)(1.0 / sqrt((double)deg)); }
+
+__global__ void __launch_bounds__(kDegThreads) degree_kernel(const int32_t* __restrict__ off, const float* __restrict__ w, int64_t n,
+                                                             int unit, float* __restrict__ dis, int* __restrict__ list,
+                                                             int* __restrict__ count) {
+    const int64_t v = (int64_t)blockIdx.x * kDegThreads + threadIdx.x;
     if (v >= n) return;
     const int32_t s = off[v], e = off[v + 1];
     float deg = 0.f;
@@ -360,10 +519,62 @@ __global__ void degree_kernel(const int32_t* __restrict__ off, const float* __re
             deg = 0.f;
             for (int32_t j = s; j < e; j++) deg = __fadd_rn(deg, 1.f);
         }
+    } else if (e - s <= kThreadColumn) {
+        for (int32_t j = s; j < e; j++) deg = __fadd_rn(deg, __ldg(w + j));
     } else {
-        for (int32_t j = s; j < e; j++) deg = __fadd_rn(deg, w[j]);
+        if (e - s <= kLongColumn) list[atomicAdd(&count[0], 1)] = (int)v;
+        else list[n - 1 - atomicAdd(&count[1], 1)] = (int)v;
+        return;
     }
-    dis[v] = (float)(1.0 / sqrt((double)deg));
+    dis[v] = inv_sqrt_degree(deg);
+}
+
+__global__ void __launch_bounds__(kDegThreads) degree_listed_kernel(const int32_t* __restrict__ off, const float* __restrict__ w,
+                                                                    int64_t n, float* __restrict__ dis, const int* __restrict__ list,
+                                                                    const int* __restrict__ count) {
+    __shared__ float s_part[kDegThreads / 32];
+    const int lane = threadIdx.x & 31;
+    const int n_warp = count[0], n_block = count[1];
+    for (int i = blockIdx.x; i < n_block; i += gridDim.x) {
+        const int64_t v = list[n - 1 - i];
+        const int64_t s = off[v], e = off[v + 1];
+        float acc[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) acc[k] = 0.f;
+        for (int64_t j = s + threadIdx.x; j < e; j += 8 * kDegThreads) {
+            float t[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) t[k] = j + k * kDegThreads < e ? __ldg(w + j + k * kDegThreads) : 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; k++) acc[k] += t[k];
+        }
+        float sum = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+#pragma unroll
+        for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+        if (lane == 0) s_part[threadIdx.x >> 5] = sum;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float deg = 0.f;
+#pragma unroll
+            for (int q = 0; q < kDegThreads / 32; q++) deg += s_part[q];
+            dis[v] = inv_sqrt_degree(deg);
+        }
+        __syncthreads();
+    }
+    const int warps = (int)gridDim.x * (kDegThreads / 32);
+    for (int i = (int)blockIdx.x * (kDegThreads / 32) + (threadIdx.x >> 5); i < n_warp; i += warps) {
+        const int v = list[i];
+        const int32_t s = off[v], e = off[v + 1];
+        float deg = 0.f;
+        float next = s + lane < e ? __ldg(w + s + lane) : 0.f;
+        for (int32_t j = s; j < e; j += 32) {
+            const float t = next;
+            next = j + 32 + lane < e ? __ldg(w + j + 32 + lane) : 0.f;
+#pragma unroll
+            for (int k = 0; k < 32; k++) deg = __fadd_rn(deg, __shfl_sync(kFull, t, k));   // + 0 beyond the column's end
+        }
+        if (lane == 0) dis[v] = inv_sqrt_degree(deg);
+    }
 }
 
 // w'[j] = (dis[source] * w[j]) * dis[destination]  (nn/conv/gcn_conv.py:37); key is the segment
@@ -540,10 +751,12 @@ struct ConvertWs {
     int32_t *key[2], *idx[2];
     float* w[2];
     int* matrix;
+    int* matrix2;     // first-pass counts of the second format, taken with the first's
     int* scan_sums;
     float* dis;
     float* loop_w;
     int* last_loop;
+    int* deg_count;      // [2] columns listed by degree_kernel
     unsigned long long* kept;
     size_t bytes;
 };
@@ -556,12 +769,14 @@ static ConvertWs carve_convert(void* ws, int64_t cap, int64_t n) {
         v.idx[b] = c.take<int32_t>(cap);
         v.w[b] = c.take<float>(cap);
     }
-    const int64_t tiles = (cap + kSortTile - 1) / kSortTile + 1;
+    const int64_t tiles = sort_tiles(cap, kItemsFew) + 1;   // the form with the most tiles
     v.matrix = c.take<int>((size_t)tiles * kRadix);
+    v.matrix2 = c.take<int>((size_t)tiles * kRadix);
     v.scan_sums = c.take<int>((size_t)((tiles + kChunkTiles - 1) / kChunkTiles + 1) * kRadix);
     v.dis = c.take<float>(n + 1);
     v.loop_w = c.take<float>(n + 1);
     v.last_loop = c.take<int>(n + 1);
+    v.deg_count = c.take<int>(2);
     v.kept = c.take<unsigned long long>(1);
     v.bytes = c.total();
     return v;
@@ -572,20 +787,28 @@ static ConvertWs carve_convert(void* ws, int64_t cap, int64_t n) {
 // element count after a first pass that drops entries, or null when first.count is exact.
 // *sorted_key receives the buffer holding the sorted keys.
 // carry_w = false (all weights are 1): out_w is left untouched, the caller fills it.
+// counted: the first pass's per-tile digit counts when the caller has them already (else null);
+// total (device, or null) receives the number of entries the first pass keeps.
 static int radix_sort(SortSrc first, int64_t n, int canonical, const unsigned long long* kept, ConvertWs& ws,
-                      int32_t* out_idx, float* out_w, int32_t** sorted_key, cudaStream_t st, bool carry_w = true) {
+                      int32_t* out_idx, float* out_w, int32_t** sorted_key, cudaStream_t st, bool carry_w = true,
+                      int* counted = nullptr, unsigned long long* total = nullptr) {
     static bool attr_set[64] = {false};
     int dev = 0;
     JG_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        JG_CUDA(cudaFuncSetAttribute(sort_scatter_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScatterSmem));
-        JG_CUDA(cudaFuncSetAttribute(sort_scatter_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScatterSmem));
+        for (int v = 0; v < 6; v++) {
+            const bool has_w = v >= 4, sorted = v & 1;
+            const int items = v >= 2 && v < 4 ? kItemsMany : kItemsFew;
+            JG_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(scatter_fn(has_w, sorted, items)),
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem(has_w, items)));
+        }
         attr_set[dev] = true;
     }
     const int bits = bits_for(n);
     const int key_passes = (bits + 7) / 8;
     const int total_passes = canonical ? 2 * key_passes : key_passes;
-    const int64_t tiles = (first.count + kSortTile - 1) / kSortTile;  // upper bound for every pass
+    const int items = sort_items(first.count, carry_w);
+    const int64_t tiles = sort_tiles(first.count, items);  // upper bound for every pass
     SortSrc src = first;
     int cur = 0;
     *sorted_key = ws.key[0];
@@ -593,18 +816,23 @@ static int radix_sort(SortSrc first, int64_t n, int canonical, const unsigned lo
     for (int p = 0; p < total_passes; p++) {
         const int from_idx = canonical && p < key_passes;
         const int shift = 8 * (canonical && !from_idx ? p - key_passes : p);
-        if (src.mode == 0)
-            sort_hist_kernel<true><<<(unsigned)tiles, kSortThreads, 0, st>>>(src, shift, from_idx, ws.matrix, tiles);
-        else
-            sort_hist_kernel<false><<<(unsigned)tiles, kSortThreads, 0, st>>>(src, shift, from_idx, ws.matrix, tiles);
-        JG_LAUNCH_CHECK();
-        {
+        int* matrix = ws.matrix;
+        if (p == 0 && counted) {
+            matrix = counted;
+        } else {
+            launch_hist(src, shift, from_idx, matrix, tiles, items, st);
+            JG_LAUNCH_CHECK();
+        }
+        if (tiles <= kChunkTiles) {
+            colscan_small<<<1, kRadix, 0, st>>>(matrix, (int)tiles, p == 0 ? total : nullptr);
+            JG_LAUNCH_CHECK();
+        } else {
             const int64_t chunks = (tiles + kChunkTiles - 1) / kChunkTiles;
-            colscan_chunk_sums<<<(unsigned)chunks, kRadix, 0, st>>>(ws.matrix, tiles, ws.scan_sums);
+            colscan_chunk_sums<<<(unsigned)chunks, kRadix, 0, st>>>(matrix, tiles, ws.scan_sums);
             JG_LAUNCH_CHECK();
-            colscan_chunks<<<1, kRadix, 0, st>>>(ws.scan_sums, chunks);
+            colscan_chunks<<<1, kRadix, 0, st>>>(ws.scan_sums, chunks, p == 0 ? total : nullptr);
             JG_LAUNCH_CHECK();
-            colscan_apply<<<(unsigned)chunks, kRadix, 0, st>>>(ws.matrix, tiles, ws.scan_sums);
+            colscan_apply<<<(unsigned)chunks, kRadix, 0, st>>>(matrix, tiles, ws.scan_sums);
             JG_LAUNCH_CHECK();
         }
         const bool last = p == total_passes - 1;
@@ -612,10 +840,7 @@ static int radix_sort(SortSrc first, int64_t n, int canonical, const unsigned lo
         dst.key = ws.key[cur];
         dst.idx = last ? out_idx : ws.idx[cur];
         dst.w = carry_w ? (last ? out_w : ws.w[cur]) : nullptr;
-        if (carry_w)
-            sort_scatter_kernel<true><<<(unsigned)tiles, kSortThreads, kScatterSmem, st>>>(src, dst, shift, from_idx, ws.matrix, tiles);
-        else
-            sort_scatter_kernel<false><<<(unsigned)tiles, kSortThreads, kScatterSmem, st>>>(src, dst, shift, from_idx, ws.matrix, tiles);
+        scatter_fn(carry_w, src.mode == 0, items)<<<(unsigned)tiles, kSortThreads, scatter_smem(carry_w, items), st>>>(src, dst, shift, from_idx, matrix);
         JG_LAUNCH_CHECK();
         *sorted_key = dst.key;
         SortSrc nxt = {};
@@ -670,7 +895,7 @@ int jg_coo_to_compressed(const int32_t* edge_index, const float* w, int64_t n_ed
         fill_int_kernel<<<blocks_for(n_edges, 256), 256, 0, st>>>(reinterpret_cast<int*>(out_w), 0x3f800000, n_edges);
         JG_LAUNCH_CHECK();
     }
-    offsets_from_sorted_keys<<<blocks_for((n_edges + 4) / 4, 256), 256, 0, st>>>(skey, n_edges, nullptr, n_nodes, out_off);
+    offsets_from_sorted_keys<<<offset_blocks(n_edges), kOffThreads, 0, st>>>(skey, n_edges, nullptr, n_nodes, out_off);
     JG_LAUNCH_CHECK();
     return JG_OK;
 }
@@ -694,13 +919,6 @@ int jg_gcn_norm_compressed(const int32_t* edge_index, const float* w, int64_t n_
     const int32_t* dst = edge_index + n_edges;
     const int grid = sm_count() * 8;
 
-    // entries that survive: non-loop input entries + one loop per node; without self-loops the list as given
-    set_count_kernel<<<1, 1, 0, st>>>(ws.kept, (unsigned long long)(add_self_loops ? n_nodes : n_edges));
-    JG_LAUNCH_CHECK();
-    if (n_edges > 0 && add_self_loops) {
-        count_kept_kernel<<<grid, 256, 0, st>>>(src, dst, n_edges, ws.kept);
-        JG_LAUNCH_CHECK();
-    }
     const bool unit = (w == nullptr) && (fill == 1.0f || !add_self_loops);
     const float* loop_w = nullptr;
     if (!unit && n_nodes > 0 && add_self_loops) {
@@ -725,13 +943,31 @@ int jg_gcn_norm_compressed(const int32_t* edge_index, const float* w, int64_t n_
     // destination-major (CSC), raw weights; degrees and dis from its segments
     int32_t* skey = nullptr;
     first.by = 1;
-    int rc = radix_sort(first, n_nodes, canonical, ws.kept, ws, csc_idx, csc_w, &skey, st, !unit);
+    int* counted = nullptr;
+    if (csr_idx && !canonical && first.count > 0) {
+        const int items = sort_items(first.count, !unit);
+        auto kern = items == kItemsFew ? sort_hist_both_kernel<kItemsFew> : sort_hist_both_kernel<kItemsMany>;
+        kern<<<(unsigned)sort_tiles(first.count, items), kHistThreads, 0, st>>>(first, ws.matrix, ws.matrix2);
+        JG_LAUNCH_CHECK();
+        counted = ws.matrix;
+    }
+    // ws.kept, the entries that survive (non-loop input entries + one loop per node; without self-loops the list as
+    // given), is the total of the first pass's counts
+    int rc = first.count > 0 ? JG_OK : launch_set_count(ws.kept, 0, st);
     if (rc != JG_OK) return rc;
-    offsets_from_sorted_keys<<<blocks_for((cap + 4) / 4, 256), 256, 0, st>>>(skey, 0, ws.kept, n_nodes, csc_off);
+    rc = radix_sort(first, n_nodes, canonical, ws.kept, ws, csc_idx, csc_w, &skey, st, !unit, counted, ws.kept);
+    if (rc != JG_OK) return rc;
+    offsets_from_sorted_keys<<<offset_blocks(cap), kOffThreads, 0, st>>>(skey, 0, ws.kept, n_nodes, csc_off);
     JG_LAUNCH_CHECK();
     if (n_nodes > 0) {
-        degree_kernel<<<blocks_for(n_nodes, 256), 256, 0, st>>>(csc_off, csc_w, n_nodes, unit ? 1 : 0, ws.dis);
+        int* list = ws.last_loop;      // free again: the loop weights have been taken
+        if (!unit) JG_CUDA(cudaMemsetAsync(ws.deg_count, 0, 2 * sizeof(int), st));
+        degree_kernel<<<blocks_for(n_nodes, kDegThreads), kDegThreads, 0, st>>>(csc_off, csc_w, n_nodes, unit ? 1 : 0, ws.dis, list, ws.deg_count);
         JG_LAUNCH_CHECK();
+        if (!unit) {
+            degree_listed_kernel<<<sm_count() * 4, kDegThreads, 0, st>>>(csc_off, csc_w, n_nodes, ws.dis, list, ws.deg_count);
+            JG_LAUNCH_CHECK();
+        }
     }
     rc = launch_norm_weights(skey, csc_idx, csc_w, ws.dis, ws.kept, 1, unit ? 1 : 0, cap, st);
     if (rc != JG_OK) return rc;
@@ -753,10 +989,10 @@ int jg_gcn_norm_compressed(const int32_t* edge_index, const float* w, int64_t n_
             weights_done = !unit;
         } else {
             first.by = 0;
-            rc = radix_sort(first, n_nodes, canonical, ws.kept, ws, csr_idx, csr_w, &skey, st, !unit);
+            rc = radix_sort(first, n_nodes, canonical, ws.kept, ws, csr_idx, csr_w, &skey, st, !unit, counted ? ws.matrix2 : nullptr);
         }
         if (rc != JG_OK) return rc;
-        offsets_from_sorted_keys<<<blocks_for((cap + 4) / 4, 256), 256, 0, st>>>(skey, 0, ws.kept, n_nodes, csr_off);
+        offsets_from_sorted_keys<<<offset_blocks(cap), kOffThreads, 0, st>>>(skey, 0, ws.kept, n_nodes, csr_off);
         JG_LAUNCH_CHECK();
         if (!weights_done) {
             rc = launch_norm_weights(skey, csr_idx, csr_w, ws.dis, ws.kept, 0, unit ? 1 : 0, cap, st);

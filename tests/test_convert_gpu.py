@@ -172,3 +172,41 @@ def test_to_undirected(cuda, oracle):
         if oracle.have_ref() and E:
             rei, _ = oracle.to_undirected(ei, a, n, "ref")       # the reference's indices (its attribute choice is unspecified)
             assert np.array_equal(host(gei), rei)
+
+
+@pytest.mark.parametrize("E", [2047, 2048, 2049, 128 * 2048, 128 * 2048 + 1, (1 << 21) - 1, 1 << 21, (1 << 21) + 4095])
+def test_tile_edges_and_entries_per_thread(cuda, oracle, E):
+    """Unit weights around one tile, the one-launch scan's last size and the step from 8 to 16 entries per thread."""
+    rng = np.random.default_rng(E)
+    n = 70001
+    ei = np.minimum((rng.random((2, E)) ** 3 * n).astype(np.int32), n - 1)
+    for by, fn, ofn in ((0, cuda.cootocsr, oracle.coo_to_csr), (1, cuda.cootocsc, oracle.coo_to_csc)):
+        got = fn(dev(ei), None, n)
+        idx, off, ow = ofn(ei, np.ones(E, np.float32), n)
+        g_idx, g_off = (got.column_indices, got.row_offset) if by == 0 else (got.row_indices, got.column_offset)
+        assert np.array_equal(host(g_off), off) and np.array_equal(host(g_idx), idx) and np.array_equal(host(got.edge_weight), ow)
+    check_gcn(cuda, oracle, ei[:, : E - E // 8], None, n)
+
+
+def test_long_weighted_columns(cuda):
+    """Columns beyond 4096 entries are summed by a block: per thread at most k / 2048 + 1 adds into eight parts, three
+    adds over the parts, five over the warp, eight over the warps.  dis halves the relative error, the other end's
+    column has at most 64 entries, and the two products and two roundings of dis add 2^-24 each."""
+    rng = np.random.default_rng(5)
+    n, hubs = 4000, [3, 300, 301, 2777, 17, 18]
+    sizes = [4095, 4096, 40961, 63, 64, 95]     # with the loop: a warp's last, a block's first, a thread's last, a warp's first
+    dst = np.concatenate([np.full(k, h) for h, k in zip(hubs, sizes)] + [rng.integers(100, 300, 2000)])
+    src = rng.integers(0, n, dst.size)
+    dst, src = np.where(src == dst, (dst + 1) % n, dst), src
+    w = (rng.random(dst.size) + 0.5).astype(np.float32)
+    csc, _ = cuda.gcn_norm_csc_csr(dev(np.stack([src, dst]).astype(np.int32)), dev(w), n)
+    off, idx, got = host(csc.column_offset), host(csc.row_indices), host(csc.edge_weight).astype(np.float64)
+    order = np.argsort(np.concatenate([dst, np.arange(n)]), kind="stable")
+    raw = np.concatenate([w, np.ones(n, np.float32)]).astype(np.float64)[order]
+    col = np.repeat(np.arange(n), np.diff(off))
+    dis = 1.0 / np.sqrt(np.bincount(col, raw, n))
+    want = dis[idx] * raw * dis[col]
+    terms = np.diff(off)
+    adds = np.where(terms <= 4096, terms, terms / 2048 + 17)
+    bound = (0.5 * (adds[idx] + adds[col]) + 6) * 2.0**-24
+    assert np.all(np.abs(got - want) <= bound * want)
