@@ -39,7 +39,8 @@ struct GemmParams {
     float* out;
     const float* bias;
     int64_t n_rows;
-    int32_t k, m;       // reduction length, output width
+    int32_t k, m;       // reduction length, output columns per column tile (grid.y of them)
+    int32_t m_total;    // output width
     int32_t m_pad;      // TMEM columns per accumulator (power of two >= 32)
     int32_t relu;
     int32_t n_tiles, k_blocks;
@@ -48,8 +49,7 @@ struct GemmParams {
     const float* wt;
     int32_t plain_loads;
     int32_t tma_store;   // epilogue stages 32x32 blocks in shared memory and stores them by TMA
-    int32_t ldo;         // row pitch of the output in floats (the full width when m is one column tile of it)
-    int32_t col_base;    // first output column of this tile (out, bias and wt already point at it)
+    int32_t ldo;         // row pitch of the output in floats
     __half* out_half;    // optional second copy of the result in fp16 (same shape and pitch in elements), or null
     uint32_t wait_spins; // limit of every mbarrier wait (kWaitSpins; the time-out test entry shortens it)
     int32_t withhold;    // time-out test entry only: the producer skips this fill of the ring (-1: none)
@@ -166,6 +166,11 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // ring first (1024-byte aligned stages), control block after it
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    // blockIdx.y: column tile, p.m wide (the last one may be narrower: col_m columns)
+    const int col0 = (int)blockIdx.y * p.m;
+    const int col_m = p.m_total - col0 < p.m ? p.m_total - col0 : p.m;
+    const float* bias = p.bias ? p.bias + col0 : nullptr;
+    const float* wt = p.wt + (int64_t)col0 * p.k;
     const uint32_t a_bytes = kTileM * kTileK * 4;                    // 16 KB
     const uint32_t b_rows = (uint32_t)((p.m + 15) / 16 * 16);   // MMA N: a multiple of 16 when M = 128
     const uint32_t b_bytes = ((b_rows * kTileK * 4) + 1023) / 1024 * 1024;
@@ -250,11 +255,11 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     }
                     {
                         const uint32_t dst = a_dst + a_bytes + lane_off;
-                        const float* src = p.wt + (int64_t)r_first * p.k + kc;
+                        const float* src = wt + (int64_t)r_first * p.k + kc;
                         const int groups = (int)b_rows / 8;
                         for (int j = 0; j < groups; j++) {
-                            const bool in = kin2 && (int)(r_first + 8 * j) < p.m;
-                            cp_async8(dst + j * 1024, in ? src + j * step : p.wt, in);
+                            const bool in = kin2 && (int)(r_first + 8 * j) < col_m;
+                            cp_async8(dst + j * 1024, in ? src + j * step : wt, in);
                         }
                     }
                     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&ctl->full[s])) : "memory");
@@ -288,13 +293,13 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 }
                 {
                     const uint32_t b_dst = a_dst + a_bytes;
-                    const float* src_even = p.wt + (int64_t)pw * p.k + kcol;
+                    const float* src_even = wt + (int64_t)pw * p.k + kcol;
                     const float* src_odd = src_even + 4 * (int64_t)p.k;
                     const int groups = (int)b_rows / 8;
                     for (int j = 0; j < groups; j++) {
-                        const bool in_e = kin && (int)(pw + 8 * j) < p.m, in_o = kin && (int)(pw + 4 + 8 * j) < p.m;
-                        cp_async4(b_dst + off_even + j * 1024, in_e ? src_even + j * step : p.wt, in_e);
-                        cp_async4(b_dst + off_odd + j * 1024, in_o ? src_odd + j * step : p.wt, in_o);
+                        const bool in_e = kin && (int)(pw + 8 * j) < col_m, in_o = kin && (int)(pw + 4 + 8 * j) < col_m;
+                        cp_async4(b_dst + off_even + j * 1024, in_e ? src_even + j * step : wt, in_e);
+                        cp_async4(b_dst + off_odd + j * 1024, in_o ? src_odd + j * step : wt, in_o);
                     }
                 }
                 asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&ctl->full[s])) : "memory");
@@ -314,7 +319,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     unsigned char* a_dst = ring + s * stage_bytes;
                     mbar_expect_tx(&ctl->full[s], a_bytes + b_rows * kTileK * 4);
                     tma_load_2d(a_dst, &map_x, kb * kTileK, tile * kTileM, &ctl->full[s]);
-                    tma_load_2d(a_dst + a_bytes, &map_w, kb * kTileK, 0, &ctl->full[s]);
+                    tma_load_2d(a_dst + a_bytes, &map_w, kb * kTileK, col0, &ctl->full[s]);
                 }
             }
         }
@@ -355,7 +360,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         // alternate 32-column chunks.
         const int quad = warp & 3;
         const int half = (warp - 2) >> 2;
-        const bool full_chunks = (p.m % 32) == 0 && (p.ldo % 4) == 0;   // 16-byte stores need 16-byte aligned row starts
+        const bool full_chunks = (col_m % 32) == 0 && (p.ldo % 4) == 0;   // 16-byte stores need 16-byte aligned row starts
         uint32_t local_tile = 0;
         for (int tile = blockIdx.x; tile < p.n_tiles && !*abort_flag; tile += gridDim.x, local_tile++) {
             const int b = local_tile & 1;
@@ -363,17 +368,17 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             tc_fence_after();
             const int64_t row = (int64_t)tile * kTileM + quad * 32 + lane;
             const uint32_t taddr = tmem_base + (uint32_t)(b * p.m_pad) + ((uint32_t)(quad * 32) << 16);
-            for (int c0 = half * 32; c0 < p.m; c0 += 64) {
+            for (int c0 = half * 32; c0 < col_m; c0 += 64) {
                 float v[32];
                 tmem_ld32(taddr + (uint32_t)c0, v, c0 + 16 < (int)b_rows);
                 if (p.tma_store) {
                     // bias / ReLU, then the warp's 32x32 block goes to its slab in the 128-byte swizzle
                     // (16-byte chunk c of row r at chunk c ^ (r & 7)) and leaves as ONE bulk tensor store:
                     // full 128-byte row segments instead of 32 scattered 16-byte stores per instruction.
-                    if (p.bias) {
+                    if (bias) {
 #pragma unroll
                         for (int i = 0; i < 32; i++)
-                            if (c0 + i < p.m) v[i] += __ldg(p.bias + c0 + i);
+                            if (c0 + i < col_m) v[i] += __ldg(bias + c0 + i);
                     }
                     if (p.relu) {
 #pragma unroll
@@ -407,18 +412,18 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     __syncwarp();
                     if (lane == 0) {
                         asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
-                                     ::"l"(&map_out), "r"(p.col_base + c0), "r"(tile * kTileM + quad * 32), "r"(smem_u32(slab)) : "memory");
+                                     ::"l"(&map_out), "r"(col0 + c0), "r"(tile * kTileM + quad * 32), "r"(smem_u32(slab)) : "memory");
                         if (p.out_half)
                             asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
-                                         ::"l"(&map_half), "r"(p.col_base + c0), "r"(tile * kTileM + quad * 32), "r"(smem_u32(hslab)) : "memory");
+                                         ::"l"(&map_half), "r"(col0 + c0), "r"(tile * kTileM + quad * 32), "r"(smem_u32(hslab)) : "memory");
                         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     }
                 } else if (row < p.n_rows) {
-                    float* o = p.out + row * p.ldo + c0;
-                    if (p.bias) {
+                    float* o = p.out + row * p.ldo + col0 + c0;
+                    if (bias) {
 #pragma unroll
                         for (int i = 0; i < 32; i++)
-                            if (full_chunks || c0 + i < p.m) v[i] += __ldg(p.bias + c0 + i);
+                            if (full_chunks || c0 + i < col_m) v[i] += __ldg(bias + c0 + i);
                     }
                     if (p.relu) {
 #pragma unroll
@@ -431,7 +436,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     } else {
 #pragma unroll
                         for (int i = 0; i < 32; i++)
-                            if (c0 + i < p.m) o[i] = v[i];
+                            if (c0 + i < col_m) o[i] = v[i];
                     }
                 }
             }
@@ -660,9 +665,9 @@ size_t jg_gemm_tf32_workspace_bytes(void) { return 256; }
 static thread_local uint32_t g_test_wait_spins = kWaitSpins;
 static thread_local int32_t g_test_withhold = -1;
 
-// One column tile (at most 256 output columns) of the product.
-static int gemm_tile(float* out, const float* x, const float* wt, const float* bias, int64_t n_rows, int64_t k, int64_t m,
-                     int64_t m_total, int64_t col_base, int relu, int32_t* error, cudaStream_t st, __half* out_half = nullptr) {
+// The product in column tiles of `m` (at most 256) of the m_total output columns, one launch.
+static int gemm_launch(float* out, const float* x, const float* wt, const float* bias, int64_t n_rows, int64_t k, int64_t m,
+                       int64_t m_total, int relu, int32_t* error, cudaStream_t st, __half* out_half = nullptr) {
     // TMA needs 16-byte aligned bases and row pitches; anything else goes through the plain-load producer
     const bool plain = (k % 4 != 0) || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(wt)) % 16 != 0);
     const int b_rows = (int)((m + 15) / 16 * 16);
@@ -672,7 +677,7 @@ static int gemm_tile(float* out, const float* x, const float* wt, const float* b
     if (!plain) {
         int rc = make_map(&map_x, x, n_rows, k, kTileM);
         if (rc != JG_OK) return rc;
-        rc = make_map(&map_w, wt, m, k, b_rows);
+        rc = make_map(&map_w, wt, m_total, k, b_rows);
         if (rc != JG_OK) return rc;
     }
     GemmParams p = {};
@@ -680,21 +685,21 @@ static int gemm_tile(float* out, const float* x, const float* wt, const float* b
     const bool pairs = (k % 2 == 0) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(wt)) % 8 == 0);
     p.x = x; p.wt = wt; p.plain_loads = plain ? (pairs ? 2 : 1) : 0;
     // TMA store needs a 16-byte row pitch for the output
-    p.tma_store = (m_total % 4 == 0 && m % 4 == 0) ? 1 : 0;
+    p.tma_store = m_total % 4 == 0 ? 1 : 0;
     CUtensorMap map_out;
     memset(&map_out, 0, sizeof(map_out));
     if (p.tma_store) {
-        int rc2 = make_map(&map_out, out - col_base, n_rows, m_total, 32);
+        int rc2 = make_map(&map_out, out, n_rows, m_total, 32);
         if (rc2 != JG_OK) return rc2;
     }
     p.out = out; p.bias = bias; p.n_rows = n_rows; p.k = (int32_t)k; p.m = (int32_t)m; p.relu = relu;
-    p.ldo = (int32_t)m_total; p.col_base = (int32_t)col_base;
+    p.ldo = (int32_t)m_total; p.m_total = (int32_t)m_total;
     p.out_half = out_half;
     CUtensorMap map_half;
     memset(&map_half, 0, sizeof(map_half));
     if (out_half) {
         JG_CHECK_ARG(p.tma_store, JG_ESHAPE, "gemm_tf32: the fp16 copy needs an output width that is a multiple of 8");
-        int rc3 = make_map_half(&map_half, out_half - col_base, n_rows, m_total);
+        int rc3 = make_map_half(&map_half, out_half, n_rows, m_total);
         if (rc3 != JG_OK) return rc3;
     }
     int pad = 32;
@@ -718,7 +723,7 @@ static int gemm_tile(float* out, const float* x, const float* wt, const float* b
     }
     int grid = sm_count();
     if (grid > p.n_tiles) grid = p.n_tiles;
-    gemm_tf32_kernel<<<grid, kGemmThreads, smem, st>>>(map_x, map_w, map_out, map_half, p);
+    gemm_tf32_kernel<<<dim3((unsigned)grid, (unsigned)((m_total + m - 1) / m)), kGemmThreads, smem, st>>>(map_x, map_w, map_out, map_half, p);
     JG_LAUNCH_CHECK();
     return JG_OK;
 }
@@ -739,16 +744,14 @@ static int gemm_impl(float* out, void* out_half, const float* x, const float* wt
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int32_t* error = static_cast<int32_t*>(workspace);
     if (clear_error) JG_CUDA(cudaMemsetAsync(error, 0, sizeof(int32_t), st));
-    // wider outputs: one launch per tile of 256 columns (x is read once per tile); 128 columns when the fp16
-    // copy needs its own staging slabs in shared memory
-    const int64_t tile_w = out_half ? 128 : 256;
-    for (int64_t cb = 0; cb < m; cb += tile_w) {
-        const int64_t mt = m - cb < tile_w ? m - cb : tile_w;
-        int rc = gemm_tile(out + cb, x, wt + cb * k, bias ? bias + cb : nullptr, n_rows, k, mt, m, cb, relu, error, st,
-                           out_half ? static_cast<__half*>(out_half) + cb : nullptr);
-        if (rc != JG_OK) return rc;
-    }
-    return JG_OK;
+    // Column tiles of 256 (128 when the fp16 copy needs its own staging slabs in shared memory), x read once per
+    // tile; halved, down to 64, while the tiles do not reach every SM: a citation graph's 2708 x 1433 -> 256 is
+    // 22 row tiles, and the time of one is set by how many rows of both operands it has to fetch per step.
+    int64_t tile_w = out_half ? 128 : 256;
+    const int64_t row_tiles = (n_rows + kTileM - 1) / kTileM;
+    while (tile_w > 64 && m > tile_w / 2 && row_tiles * ((m + tile_w - 1) / tile_w) < sm_count()) tile_w /= 2;
+    if (tile_w > m) tile_w = m;
+    return gemm_launch(out, x, wt, bias, n_rows, k, tile_w, m, relu, error, st, static_cast<__half*>(out_half));
 }
 
 int jg_gemm_tf32(float* out, const float* x, const float* wt, const float* bias, int64_t n_rows, int64_t k, int64_t m,

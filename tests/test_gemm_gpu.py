@@ -241,3 +241,21 @@ def test_fp32_row_reduction_tile_edges(cuda, M, N, K):
     scale = a.double().abs().t() @ b.double().abs()
     assert ((got.double() - want).abs() <= 130 * 2.0**-24 * scale).all()
     assert torch.equal(got, cuda.ops.matmul_f32(a, b, trans_a=True))
+
+
+@pytest.mark.parametrize("m", [47, 65, 100, 130, 256, 300])
+@pytest.mark.parametrize("k", [33, 64, 602])
+def test_column_tiles_of_short_inputs(cuda, k, m):
+    """With few rows the output is cut into column tiles of 64 or 128; every value is the same sum as in the one-tile
+    product of the same rows among many."""
+    g = torch.Generator(device="cuda").manual_seed(k + m)
+    x = torch.randn((40000, k), device="cuda", generator=g)
+    w = torch.randn((k, m), device="cuda", generator=g)
+    bias = torch.randn(m, device="cuda", generator=g)
+    many = cuda.ops.linear_tf32(x, w, bias=bias, relu=True)
+    for n in (1, 200, 5000):
+        few = cuda.ops.linear_tf32(x[:n].contiguous(), w, bias=bias, relu=True, check_status=True)
+        assert torch.equal(few, many[:n])
+    want = torch.relu(x.double() @ w.double() + bias.double())
+    scale = x.abs().double() @ w.abs().double() + bias.abs().double()
+    assert ((many.double() - want).abs() / scale).max().item() <= 2e-3
