@@ -88,6 +88,8 @@ SIGNATURES = {
     "jg_gemm_tn_tf32": (ctypes.c_int, [vp, vp, vp, i64, i64, i64, vp, vp, sz, vp]),
     "jg_gemm_f32_workspace_bytes": (sz, [i64, i64, i64]),
     "jg_gemm_f32": (ctypes.c_int, [vp, vp, vp, vp, i64, i64, i64, i64, i64, i64, i64, i64, ctypes.c_int, vp, sz, vp]),
+    "jg_relu_grad_workspace_bytes": (sz, [i64, i64]),
+    "jg_relu_grad_f32": (ctypes.c_int, [vp, vp, vp, vp, i64, i64, vp, sz, vp]),
     "jg_aggregate_static_capacity_bytes": (sz, []),
     "jg_aggregate_f32_static": (ctypes.c_int, [vp, vp, vp, vp, vp, i64, i64, i64, i64, vp]),
 }

@@ -191,6 +191,21 @@ def aggregateWithWeight(x, csc, csr, weight=None):
     return _AggregateFunc.apply(x, csc, csr, weight)
 
 
+def _epilogue_grad(grad, out, want_sum):
+    """``(grad * (out > 0), its column sums)``: the gradient through a fused ReLU and of the bias before it, in one
+    pass.  ``out=None``: no ReLU, ``grad`` itself comes back.  The sums are ``None`` unless asked for."""
+    g = _as_f32(grad, "grad")
+    n, f = g.shape
+    y = None if out is None else _as_f32(out, "out")
+    gm = g if y is None else torch.empty_like(g)
+    gsum = torch.empty(f, dtype=torch.float32, device=g.device) if want_sum else None
+    if y is not None or want_sum:
+        ws = workspace(lib().jg_relu_grad_workspace_bytes(n, f) if want_sum else 0, g.device)
+        check(lib().jg_relu_grad_f32(None if y is None else ptr(gm), ptr(gsum), ptr(g), ptr(y), n, f, ptr(ws), ws.numel(),
+                                     stream_for(g)), "jg_relu_grad_f32")
+    return gm, gsum
+
+
 class _AggregateBiasAct(torch.autograd.Function):
     """``act(A x + b)`` with the epilogue fused into the aggregation's store; backward masks the
     gradient with the saved output, sums it for the bias and aggregates it over the CSR."""
@@ -206,17 +221,19 @@ class _AggregateBiasAct(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_output):
-        g = grad_output
-        if ctx.relu:
-            (out,) = ctx.saved_tensors
-            g = g * (out > 0)
-        g = g.contiguous()
+        out = ctx.saved_tensors[0] if ctx.relu else None
+        want_sum = ctx.has_bias and ctx.needs_input_grad[1]
         csr = ctx.csr
         gx = None
+        if ctx.needs_input_grad[0] and not (torch.is_grad_enabled() and grad_output.requires_grad):
+            g, gb = _epilogue_grad(grad_output, out, want_sum)
+        else:     # differentiable once more (create_graph), or the bias alone is trained
+            g = grad_output if out is None else grad_output * (out > 0)
+            gb = g.sum(0) if want_sum else None
+            g = g.contiguous()
         if ctx.needs_input_grad[0]:
             gx = segment_aggregate(g, csr.column_indices, csr.row_offset, csr.edge_weight,
                                    plan=_plan_of(csr, csr.row_offset, csr.column_indices.numel()))
-        gb = g.sum(0) if ctx.has_bias and ctx.needs_input_grad[1] else None
         return gx, gb, None, None, None
 
 
@@ -715,7 +732,7 @@ class _LinearF32(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_output):
         x, weight, out = ctx.saved_tensors
-        g = _relu_mask(grad_output, out) if ctx.relu else grad_output.contiguous()
+        g = _epilogue_grad(grad_output, out if ctx.relu else None, False)[0]
         gx = matmul_f32(g, weight, trans_b=True) if ctx.needs_input_grad[0] else None
         gw = matmul_f32(x, g, trans_a=True) if ctx.needs_input_grad[1] else None
         return gx, gw, None
@@ -782,11 +799,6 @@ def linear_nt(x, weight, bias=None, tf32=True):
     return _LinearNT.apply(_as_f32(x, "x"), _as_f32(weight, "weight"), bias, bool(tf32))
 
 
-def _relu_mask(grad, out):
-    """``grad * (out > 0)``: the gradient through a fused ReLU, from the saved output."""
-    return (grad * (out > 0)).contiguous()
-
-
 class _LinearTF32(torch.autograd.Function):
     """``act(x @ weight)`` through the tcgen05 kernel with a backward: ``grad_x = g @ weight^T`` runs
     on the same kernel (its transposed operand is the weight itself); ``grad_weight = x^T @ g`` is a
@@ -803,7 +815,7 @@ class _LinearTF32(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_output):
         x, weight, out = ctx.saved_tensors
-        g = _relu_mask(grad_output, out) if ctx.relu else grad_output.contiguous()
+        g = _epilogue_grad(grad_output, out if ctx.relu else None, False)[0]
         gx = gw = None
         if ctx.needs_input_grad[0]:
             if linear_tf32_supported(g.shape[0], g.shape[1], weight.shape[0]):

@@ -259,3 +259,20 @@ def test_column_tiles_of_short_inputs(cuda, k, m):
     want = torch.relu(x.double() @ w.double() + bias.double())
     scale = x.abs().double() @ w.abs().double() + bias.abs().double()
     assert ((many.double() - want).abs() / scale).max().item() <= 2e-3
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 5000])
+@pytest.mark.parametrize("f", [1, 3, 47, 64, 256, 300, 1030])
+def test_masked_gradient_and_column_sums(cuda, n, f):
+    """The epilogue's gradient: the mask is exact (a NaN stays one), a column's sum passes at most n + 8 additions."""
+    g = torch.Generator(device="cuda").manual_seed(n + f)
+    grad, y = (torch.randn((n, f), device="cuda", generator=g) for _ in range(2))
+    gm, gsum = cuda.ops._epilogue_grad(grad, y, True)
+    want = grad * (y > 0)
+    assert torch.equal(gm, want)
+    assert ((gsum.double() - want.double().sum(0)).abs() <= (n + 8) * 2.0**-24 * want.double().abs().sum(0)).all()
+    plain, total = cuda.ops._epilogue_grad(grad, None, True)
+    assert plain is grad and ((total.double() - grad.double().sum(0)).abs() <= (n + 8) * 2.0**-24 * grad.double().abs().sum(0)).all()
+    grad[0, 0], y[0, 0] = float("inf"), -1.0
+    gm, gsum = cuda.ops._epilogue_grad(grad, y, True)
+    assert torch.isnan(gm[0, 0]) and torch.isnan(gsum[0])
