@@ -34,6 +34,7 @@ SIGNATURES = {
     "jg_aggregate_add_f32": (ctypes.c_int, [vp, vp, vp, vp, vp, i64, i64, i64, i64, vp, i32, vp, sz, vp]),
     "jg_aggregate_ordered_f32": (ctypes.c_int, [vp, vp, vp, vp, vp, i64, i64, i64, i64, vp, i32, vp, sz, vp]),
     "jg_aggregate_bias_act_f32": (ctypes.c_int, [vp, vp, vp, vp, vp, vp, ctypes.c_int, i64, i64, i64, i64, vp, i32, vp, sz, vp]),
+    "jg_aggregate_combine_f32": (ctypes.c_int, [vp, vp, vp, vp, vp, vp, f32, f32, i64, i64, i64, i64, vp, i32, vp, sz, vp]),
     "jg_aggregate_opts_f32": (ctypes.c_int, [vp, vp, vp, vp, vp, vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                              i64, i64, i64, i64, vp, i32, vp, sz, vp]),
     "jg_halo_flag_bytes": (sz, []),

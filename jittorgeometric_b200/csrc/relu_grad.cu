@@ -10,7 +10,7 @@
 // A block takes consecutive rows; a thread owns V = 4 or 1 neighbouring columns and every TY-th row, four rows in
 // flight, in four accumulators.  Blocks' sums are added in a fixed order by the slice reduction: no atomics,
 // identical results run to run.
-// 170 k x 256: 0.29 ms (compare, multiply, column sum) before, 0.10 ms here.
+// 170 k x 256: 0.29 ms (compare, multiply, column sum) before, 0.13 ms here.
 #include "common.cuh"
 
 namespace jg {

@@ -98,6 +98,8 @@ struct AggArgs {
     int accumulate;  // 1: add the aggregated row to what `out` already holds (old + sum)
     int64_t max_items;  // host-side upper bound on the plan's pieces (sizes the grid)
     const float* bias;  // epilogue on finished output rows: + bias[column] (null: none) ...
+    const float* addend;  // [n_out, f] combined with the sum before the bias (null: none): scale * sum + add_scale * addend
+    float scale, add_scale;
     int relu;           // ... then max(., 0)
     int ordered;        // 1: every row must be summed in stored order (no lane groups taking alternate entries)
     int reserve_ctas;   // CTA slots of the persistent grid left free for a kernel that runs beside this one
@@ -105,8 +107,16 @@ struct AggArgs {
 };
 
 
-// Exact mode rounds multiply and add separately, as the reference CPU loop does; the fused
-// mode uses one FMA per term.
+// Exact mode rounds multiply and add separately, as the reference CPU loop does (scalar instructions: the packed
+// pair of mul.rn and add.rn comes back fused); the fused mode uses one FMA per term, two terms per instruction -
+// at the widths that use it the kernels are bound by instruction issue, and a packed FMA rounds as two scalar ones.
+__device__ __forceinline__ void fma_pair(float& a0, float& a1, float v0, float v1, unsigned long long ww) {
+    unsigned long long a, v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(a0), "f"(a1));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(v0), "f"(v1));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a) : "l"(v), "l"(ww));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(a));
+}
 template <bool EXACT>
 __device__ __forceinline__ void axpy4(float4& a, const float4& v, float w) {
     if (EXACT) {
@@ -115,31 +125,56 @@ __device__ __forceinline__ void axpy4(float4& a, const float4& v, float w) {
         a.z = __fadd_rn(__fmul_rn(v.z, w), a.z);
         a.w = __fadd_rn(__fmul_rn(v.w, w), a.w);
     } else {
-        a.x = fmaf(v.x, w, a.x);
-        a.y = fmaf(v.y, w, a.y);
-        a.z = fmaf(v.z, w, a.z);
-        a.w = fmaf(v.w, w, a.w);
+        unsigned long long ww;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "f"(w));
+        fma_pair(a.x, a.y, v.x, v.y, ww);
+        fma_pair(a.z, a.w, v.z, v.w, ww);
     }
 }
 
-// Vector-width kernel (F = 4*G*VPL).  G lanes cover one feature row, 32/G entries are gathered
-// side by side, B steps per batch.
-// EPI compiles in the bias/ReLU epilogue (a separate instantiation, so the plain kernel is untouched).
-// FULL: the row is exactly 4*G*VPL floats wide (everything about the width folds at compile time).
+// Epilogue of a finished output element: scale * sum + add_scale * addend, + bias, ReLU (each if asked for).
+__device__ __forceinline__ float finish_value(const AggArgs& a, float v, size_t at, int64_t col) {
+    if (a.addend) v = fmaf(a.scale, v, __fmul_rn(a.add_scale, __ldg(a.addend + at)));
+    if (a.bias) v += __ldg(a.bias + col);
+    if (a.relu) v = fmaxf(v, 0.f);
+    return v;
+}
+// What a kernel instantiation compiles in: nothing, bias and ReLU, or the sum with the addend.
+enum Epilogue { kPlain = 0, kBiasAct = 1, kCombine = 2 };
+template <int EPI>
+__device__ __forceinline__ float4 finish_value4(const AggArgs& a, float4 v, size_t at, int col) {
+    if (EPI == kCombine) {
+        const float4 h = __ldg(reinterpret_cast<const float4*>(a.addend + at));
+        v.x = fmaf(a.scale, v.x, __fmul_rn(a.add_scale, h.x)); v.y = fmaf(a.scale, v.y, __fmul_rn(a.add_scale, h.y));
+        v.z = fmaf(a.scale, v.z, __fmul_rn(a.add_scale, h.z)); v.w = fmaf(a.scale, v.w, __fmul_rn(a.add_scale, h.w));
+    }
+    if (EPI == kBiasAct) {
+        if (a.bias) {
+            const float4 b4 = __ldg(reinterpret_cast<const float4*>(a.bias + col));
+            v.x += b4.x; v.y += b4.y; v.z += b4.z; v.w += b4.w;
+        }
+        if (a.relu) {
+            v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f); v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f);
+        }
+    }
+    return v;
+}
+
+// Row-by-row kernel of the widths above 64 (F <= 128*VPL): the warp covers one feature row, B rows are gathered per
+// batch, entries are added in stored order.
+// EPI compiles in an epilogue (instantiations of their own: the registers of one cost the others 3 %).
+// FULL: the row is exactly 128*VPL floats wide (everything about the width folds at compile time).
 // !FULL: any 16-byte-aligned width up to that; lanes whose columns lie beyond it sit out.
-template <int G, int VPL, int B, int MINB, bool EXACT, bool EPI, bool FULL>
+template <int VPL, int B, int MINB, int EPI, bool FULL>
 __global__ void __launch_bounds__(kBlock, MINB) aggregate_rows_kernel(AggArgs a) {
-    constexpr int EPS = 32 / G;
-    const int F = FULL ? 4 * G * VPL : (int)a.f;
+    const int F = FULL ? 128 * VPL : (int)a.f;
     __shared__ int2 s_tile[kBlock / 32][32];
     const int lane = lane_id();
-    const int sub = lane / G;
-    const int fl = lane % G;
     bool qok[VPL];
 #pragma unroll
-    for (int q = 0; q < VPL; q++) qok[q] = FULL || (fl + q * G) * 4 < F;
+    for (int q = 0; q < VPL; q++) qok[q] = FULL || (lane + q * 32) * 4 < F;
     int2* tile = s_tile[threadIdx.x / 32];
-    const char* xb = reinterpret_cast<const char*>(a.x) + fl * 16;
+    const char* xb = reinterpret_cast<const char*>(a.x) + lane * 16;
     const int64_t n_items = a.hdr ? a.hdr->n_items : 0;
     const int chunk = a.hdr ? a.hdr->chunk : 0x7fffffff;
     const int64_t total = n_items + a.n_out;
@@ -214,91 +249,244 @@ __global__ void __launch_bounds__(kBlock, MINB) aggregate_rows_kernel(AggArgs a)
                 __syncwarp();
                 const int cnt = min(32, e - j0);
                 int t = 0;
-                for (; t + EPS * B <= cnt; t += EPS * B) {  // full batches: no predicates
+                for (; t + B <= cnt; t += B) {  // full batches: no predicates
                     float4 v[B][VPL];
                     float wv[B];
 #pragma unroll
                     for (int u = 0; u < B; u++) {
-                        const int2 p = tile[t + u * EPS + sub];
+                        const int2 p = tile[t + u];
                         wv[u] = __int_as_float(p.y);
                         const float4* g = reinterpret_cast<const float4*>(xb + (size_t)(unsigned)p.x * (size_t)(F * 4));
 #pragma unroll
-                        for (int q = 0; q < VPL; q++) v[u][q] = qok[q] ? __ldg(g + q * G) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        for (int q = 0; q < VPL; q++) v[u][q] = qok[q] ? __ldg(g + q * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
 #pragma unroll
                     for (int u = 0; u < B; u++)
 #pragma unroll
-                        for (int q = 0; q < VPL; q++) axpy4<EXACT>(acc[q], v[u][q], wv[u]);
+                        for (int q = 0; q < VPL; q++) axpy4<true>(acc[q], v[u][q], wv[u]);
                 }
                 if (t < cnt) {  // last, partial batch
-                    // Four or more entries per step (rows of at most 32 columns): steps whose entries all lie beyond the
-                    // row are skipped by a warp-uniform test - most rows of a power-law graph are shorter than one
-                    // step, and for them seven of the eight steps are empty (F = 32: -6 % time).  With one or two
-                    // entries per step the same test measured 5 % SLOWER (it breaks up the batch of loads), so it is
-                    // compiled in for the narrow instantiation only.
                     float4 v[B][VPL];
                     float wv[B];
 #pragma unroll
                     for (int u = 0; u < B; u++) {
-                        const int k = t + u * EPS + sub;
+                        const int k = t + u;
                         wv[u] = 0.f;
 #pragma unroll
                         for (int q = 0; q < VPL; q++) v[u][q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if ((EPS < 4 || t + u * EPS < cnt) && k < cnt) {
+                        if (k < cnt) {
                             const int2 p = tile[k];
                             wv[u] = __int_as_float(p.y);
                             const float4* g = reinterpret_cast<const float4*>(xb + (size_t)(unsigned)p.x * (size_t)(F * 4));
 #pragma unroll
                             for (int q = 0; q < VPL; q++)
-                                if (qok[q]) v[u][q] = __ldg(g + q * G);
+                                if (qok[q]) v[u][q] = __ldg(g + q * 32);
                         }
                     }
 #pragma unroll
-                    for (int u = 0; u < B; u++) {
-                        if (EPS < 4 || t + u * EPS < cnt) {
+                    for (int u = 0; u < B; u++)
 #pragma unroll
-                            for (int q = 0; q < VPL; q++) axpy4<EXACT>(acc[q], v[u][q], wv[u]);
-                        }
-                    }
+                        for (int q = 0; q < VPL; q++) axpy4<true>(acc[q], v[u][q], wv[u]);
                 }
             }
-            if (EPS > 1) {
-#pragma unroll
-                for (int o = G; o < 32; o <<= 1)
-#pragma unroll
-                    for (int q = 0; q < VPL; q++) {
-                        acc[q].x += __shfl_xor_sync(kFull, acc[q].x, o);
-                        acc[q].y += __shfl_xor_sync(kFull, acc[q].y, o);
-                        acc[q].z += __shfl_xor_sync(kFull, acc[q].z, o);
-                        acc[q].w += __shfl_xor_sync(kFull, acc[q].w, o);
-                    }
-            }
-            if (sub == 0) {
-                float4* o = reinterpret_cast<float4*>(dst) + fl;
+            {
+                float4* o = reinterpret_cast<float4*>(dst) + lane;
 #pragma unroll
                 for (int q = 0; q < VPL; q++) {
                     if (!qok[q]) continue;
                     if (add_old) {
-                        const float4 old = o[q * G];
+                        const float4 old = o[q * 32];
                         acc[q].x = __fadd_rn(old.x, acc[q].x);
                         acc[q].y = __fadd_rn(old.y, acc[q].y);
                         acc[q].z = __fadd_rn(old.z, acc[q].z);
                         acc[q].w = __fadd_rn(old.w, acc[q].w);
                     }
-                    if (EPI && id >= n_items) {   // a finished output row (pieces of hub rows get theirs in the fix-up)
-                        if (a.bias) {
-                            const float4 b4 = __ldg(reinterpret_cast<const float4*>(a.bias) + fl + q * G);
-                            acc[q].x += b4.x; acc[q].y += b4.y; acc[q].z += b4.z; acc[q].w += b4.w;
-                        }
-                        if (a.relu) {
-                            acc[q].x = fmaxf(acc[q].x, 0.f); acc[q].y = fmaxf(acc[q].y, 0.f);
-                            acc[q].z = fmaxf(acc[q].z, 0.f); acc[q].w = fmaxf(acc[q].w, 0.f);
-                        }
-                    }
-                    __stcs(o + q * G, acc[q]);
+                    if (EPI != kPlain && id >= n_items)   // a finished output row (pieces of hub rows get theirs in the fix-up)
+                        acc[q] = finish_value4<EPI>(a, acc[q], (size_t)(id - n_items) * F + 4 * (lane + q * 32), 4 * (lane + q * 32));
+                    __stcs(o + q * 32, acc[q]);
                 }
             }
         }
+    }
+}
+
+// Streaming kernel of the widths up to 64.  G lanes (8 or 16) cover one feature row of F = 32 or 36 to 64 floats, 32/G
+// entries of a row are gathered side by side (one "step").  EPI compiles in the epilogue (a separate
+// instantiation, so the plain kernel is untouched).  The width is a template parameter: with it in a register the
+// 40-column form was slower than the 64-column one.
+//
+// The segments of a ticket (rows, pieces of hub rows) are walked as ONE stream of entries, each segment padded to
+// whole steps: a window of 32 stream positions at a time is looked up by the lanes (position -> segment by a
+// search over the ticket's prefix lengths), staged in shared memory as (index, weight) pairs and marked where a
+// segment ends.  Batches of B steps are double-buffered in registers across row ends, so the gathers of the next
+// rows are in flight while a row is summed and stored; walked row by row, a row of a dozen entries cost two or
+// three exposed memory latencies.  The next ticket, and its segments' bounds, are fetched while this one is walked.
+template <int F, int B, int MINB, int EPI>
+__global__ void __launch_bounds__(kBlock, MINB) aggregate_stream_kernel(AggArgs a) {
+    constexpr int G = F <= 32 ? 8 : 16;
+    constexpr int EPS = 32 / G;
+    constexpr int NBW = 32 / (EPS * B);      // batches per window of 32 stream positions
+    static_assert(F % 4 == 0 && F <= 4 * G && NBW >= 1 && NBW * EPS * B == 32, "a window holds whole batches");
+    static_assert(kGrab <= 8, "the segment search takes three steps");
+    __shared__ int2 s_tile[kBlock / 32][2][32];
+    const int lane = lane_id();
+    const int sub = lane / G;
+    const int fl = lane % G;
+    const bool mine = fl * 4 < F;    // this lane holds columns of a row
+    int2(*tile)[32] = s_tile[threadIdx.x / 32];
+    const char* xb = reinterpret_cast<const char*>(a.x) + fl * 16;
+    const int64_t n_items = a.hdr ? a.hdr->n_items : 0;
+    const int chunk = a.hdr ? a.hdr->chunk : 0x7fffffff;
+    const int64_t total = n_items + a.n_out;
+    const int grab = a.grab;
+
+    // lane i's segment of the ticket: first entry and length (-1: none, a hub row is walked as pieces)
+    auto load_segments = [&](int64_t base, int& s, int& len) {
+        s = 0; len = -1;
+        const int64_t id = base + lane;
+        if (lane < grab && id < total) {
+            if (id < n_items) {
+                const int h = a.item_hub[id], k = a.item_k[id];
+                const int row = a.hub_row[h];
+                s = a.off[row] + k * chunk;
+                len = min(a.off[row + 1] - s, chunk);
+            } else {
+                const int64_t row = id - n_items;
+                s = a.off[row];
+                len = a.off[row + 1] - s;
+                if (len > chunk) len = -1;
+            }
+        }
+    };
+    auto take = [&]() -> unsigned long long { return lane == 0 ? atomicAdd(a.ticket, (unsigned long long)grab) : 0ull; };
+
+    int64_t base = (int64_t)__shfl_sync(kFull, take(), 0);
+    if (base >= total) return;
+    int seg_s, seg_len;
+    load_segments(base, seg_s, seg_len);
+    unsigned long long coming = take();
+    for (;;) {
+        const int64_t next_base = (int64_t)__shfl_sync(kFull, coming, 0);
+        int nxt_s, nxt_len;
+        load_segments(next_base, nxt_s, nxt_len);
+        if (next_base < total) coming = take();
+
+        const int padded = seg_len > 0 ? (seg_len + EPS - 1) / EPS * EPS : 0;
+        int incl = padded;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const int t = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += t;
+        }
+        const int T = __shfl_sync(kFull, incl, 7);
+        const int excl = incl - padded;
+        unsigned todo = __ballot_sync(kFull, seg_len > 0);
+
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        // stores segment `seg` and clears the accumulators
+        auto flush = [&](int seg) {
+            const int64_t id = base + seg;
+            const bool row = id >= n_items;     // else a piece: its partial row, finished by the fix-up
+#pragma unroll
+            for (int o = G; o < 32; o <<= 1) {
+                acc.x += __shfl_xor_sync(kFull, acc.x, o);
+                acc.y += __shfl_xor_sync(kFull, acc.y, o);
+                acc.z += __shfl_xor_sync(kFull, acc.z, o);
+                acc.w += __shfl_xor_sync(kFull, acc.w, o);
+            }
+            if (sub == 0 && mine) {
+                float4* o = reinterpret_cast<float4*>(row ? a.out + (size_t)(id - n_items) * F
+                                                          : a.partial + (size_t)(a.hub_first[a.item_hub[id]] + a.item_k[id]) * F) + fl;
+                if (row && a.accumulate) {
+                    const float4 old = *o;
+                    acc.x = __fadd_rn(old.x, acc.x);
+                    acc.y = __fadd_rn(old.y, acc.y);
+                    acc.z = __fadd_rn(old.z, acc.z);
+                    acc.w = __fadd_rn(old.w, acc.w);
+                }
+                if (EPI != kPlain && row) acc = finish_value4<EPI>(a, acc, (size_t)(id - n_items) * F + 4 * fl, 4 * fl);
+                __stcs(o, acc);
+            }
+            acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        for (unsigned empty = __ballot_sync(kFull, seg_len == 0); empty; empty &= empty - 1) flush(__ffs(empty) - 1);
+
+        if (T > 0) {
+            int pf_idx, pf_w;
+            bool pf_last;
+            // this lane's position of the window that starts at p0
+            auto fetch = [&](int p0) {
+                const int p = p0 + lane;
+                pf_idx = -1; pf_w = 0; pf_last = false;
+                if (p0 >= T) return;
+                int g = 0;
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1)
+                    if (p >= __shfl_sync(kFull, incl, g + o - 1)) g += o;
+                const int q = p - __shfl_sync(kFull, excl, g);
+                const int len = __shfl_sync(kFull, seg_len, g), s = __shfl_sync(kFull, seg_s, g);
+                const int pad = __shfl_sync(kFull, padded, g);
+                if (p < T) {
+                    if (q < len) {
+                        pf_idx = ld_stream(a.idx + s + q);
+                        pf_w = __float_as_int(ld_stream(a.w + s + q));
+                    }
+                    pf_last = q == pad - 1;
+                }
+            };
+            unsigned ends0 = 0, ends1 = 0;    // window positions that end a segment, by window parity
+            auto stage = [&](int window) {
+                __syncwarp();
+                tile[window & 1][lane] = make_int2(pf_idx, pf_w);
+                const unsigned m = __ballot_sync(kFull, pf_last);
+                if (window & 1) ends1 = m; else ends0 = m;
+                __syncwarp();
+                fetch(32 * (window + 1));
+            };
+            auto issue = [&](float4 (&v)[B], int bi) {
+                const int2* t = tile[(bi / NBW) & 1] + (bi % NBW) * (B * EPS) + sub;
+#pragma unroll
+                for (int u = 0; u < B; u++) {
+                    const int src = t[u * EPS].x;
+                    v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (src >= 0 && mine) v[u] = __ldg(reinterpret_cast<const float4*>(xb + (size_t)(unsigned)src * (size_t)(F * 4)));
+                }
+            };
+            auto consume = [&](float4 (&v)[B], int bi) {
+                const int w = bi / NBW, first = (bi % NBW) * (B * EPS);
+                const int2* t = tile[w & 1] + first + sub;
+                const unsigned ends = ((w & 1) ? ends1 : ends0) >> first;
+#pragma unroll
+                for (int u = 0; u < B; u++) {
+                    axpy4<false>(acc, v[u], __int_as_float(t[u * EPS].y));
+                    if ((ends >> (u * EPS)) & ((1u << EPS) - 1u)) {
+                        flush(__ffs(todo) - 1);
+                        todo &= todo - 1;
+                    }
+                }
+            };
+            const int n_batches = (T + B * EPS - 1) / (B * EPS);
+            float4 v0[B], v1[B];
+            fetch(0);
+            stage(0);
+            issue(v0, 0);
+            for (int bi = 0; bi < n_batches; bi += 2) {
+                if (bi + 1 < n_batches) {
+                    if ((bi + 1) % NBW == 0) stage((bi + 1) / NBW);
+                    issue(v1, bi + 1);
+                }
+                consume(v0, bi);
+                if (bi + 1 >= n_batches) break;
+                if (bi + 2 < n_batches) {
+                    if ((bi + 2) % NBW == 0) stage((bi + 2) / NBW);
+                    issue(v0, bi + 2);
+                }
+                consume(v1, bi + 1);
+            }
+        }
+        if (next_base >= total) break;
+        base = next_base;
+        seg_s = nxt_s; seg_len = nxt_len;
     }
 }
 
@@ -344,11 +532,9 @@ __device__ __forceinline__ void warp_segment_any(const AggArgs& a, int32_t s, in
         for (int q = 0; q < Q; q++)
             if (c0 + q * 32 + lane < F) {
                 float v = add_old ? __fadd_rn(dst[c0 + q * 32 + lane], acc[q]) : acc[q];
-                if (final_row) {
-                    if (a.bias) v += __ldg(a.bias + c0 + q * 32 + lane);
-                    if (a.relu) v = fmaxf(v, 0.f);
-                }
-                dst[c0 + q * 32 + lane] = v;
+                const int64_t col = c0 + q * 32 + lane;
+                if (final_row) v = finish_value(a, v, (size_t)(dst - a.out) + col, col);
+                dst[col] = v;
             }
     }
 }
@@ -487,8 +673,7 @@ __global__ void __launch_bounds__(kBlock) aggregate_narrow_kernel(AggArgs a) {
                 float v = acc;
                 if (final_row) {
                     if (a.accumulate) v = __fadd_rn(dst[c], v);
-                    if (a.bias) v += __ldg(a.bias + c);
-                    if (a.relu) v = fmaxf(v, 0.f);
+                    v = finish_value(a, v, (size_t)(dst - a.out) + c, c);
                 }
                 dst[c] = v;
             }
@@ -496,25 +681,70 @@ __global__ void __launch_bounds__(kBlock) aggregate_narrow_kernel(AggArgs a) {
     }
 }
 
-// Adds the partial rows of every hub in piece order and writes the hub's output row: one thread per
-// (hub, column), consecutive threads on consecutive columns.
+// Adds the partial rows of every hub and writes the hub's output row.  A block takes a run of hubs: their rows, piece
+// counts and first slots are read side by side, then hubs of up to kFewPieces pieces are summed with one thread per
+// (hub, column), all pieces in flight, and the others one by one by the whole block, eight warps each adding an eighth
+// of the pieces in order and the eighths in order.  With one thread per (hub, column) whatever the pieces, the
+// longest hub's chain of loads was the kernel: 17 us beside a 160 us aggregation of 4.9 M entries (70 pieces).
+constexpr int kFewPieces = 8;
 __global__ void __launch_bounds__(kBlock) hub_fixup_kernel(AggArgs a) {
-    const int64_t n_hubs = a.hdr->n_hubs;
+    __shared__ int s_row[kBlock], s_first[kBlock], s_pieces[kBlock];
+    __shared__ float s_sum[kBlock / 32][32];
+    const int n_hubs = a.hdr->n_hubs;
     const int chunk = a.hdr->chunk;
-    const int64_t F = a.f;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n_hubs * F; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t h = t / F, c = t - h * F;
-        const int row = a.hub_row[h];
-        const int deg = a.off[row + 1] - a.off[row];
-        const int pieces = (deg + chunk - 1) / chunk;
-        const float* p = a.partial + (size_t)a.hub_first[h] * F + c;
-        float acc = p[0];
-        for (int k = 1; k < pieces; k++) acc = __fadd_rn(acc, p[(size_t)k * F]);
-        float* o = a.out + (size_t)row * F + c;
-        float v = a.accumulate ? __fadd_rn(*o, acc) : acc;
-        if (a.bias) v += __ldg(a.bias + c);
-        if (a.relu) v = fmaxf(v, 0.f);
-        *o = v;
+    const int F = (int)a.f;
+    const int lane = lane_id(), warp = threadIdx.x / 32;
+    int per_block = (n_hubs + (int)gridDim.x - 1) / (int)gridDim.x;
+    if (per_block > kBlock) per_block = kBlock;
+    for (int64_t h0 = (int64_t)blockIdx.x * per_block; h0 < n_hubs; h0 += (int64_t)gridDim.x * per_block) {
+        const int cnt = n_hubs - h0 < per_block ? (int)(n_hubs - h0) : per_block;
+        __syncthreads();
+        if ((int)threadIdx.x < cnt) {
+            const int row = a.hub_row[h0 + threadIdx.x];
+            s_row[threadIdx.x] = row;
+            s_first[threadIdx.x] = a.hub_first[h0 + threadIdx.x];
+            s_pieces[threadIdx.x] = (a.off[row + 1] - a.off[row] + chunk - 1) / chunk;
+        }
+        __syncthreads();
+        for (int t = threadIdx.x; t < cnt * F; t += kBlock) {
+            const int h = t / F, c = t - h * F;
+            const int pieces = s_pieces[h];
+            if (pieces > kFewPieces) continue;
+            const float* p = a.partial + (size_t)s_first[h] * F + c;
+            float v[kFewPieces];
+#pragma unroll
+            for (int k = 0; k < kFewPieces; k++) v[k] = k < pieces ? __ldg(p + (size_t)k * F) : 0.f;
+            float acc = v[0];
+#pragma unroll
+            for (int k = 1; k < kFewPieces; k++)
+                if (k < pieces) acc = __fadd_rn(acc, v[k]);
+            float* o = a.out + (size_t)s_row[h] * F + c;
+            *o = finish_value(a, a.accumulate ? __fadd_rn(*o, acc) : acc, (size_t)s_row[h] * F + c, c);
+        }
+        for (int h = 0; h < cnt; h++) {
+            const int pieces = s_pieces[h];
+            if (pieces <= kFewPieces) continue;
+            const int per = (pieces + kBlock / 32 - 1) / (kBlock / 32);
+            const int k0 = warp * per, k1 = k0 + per < pieces ? k0 + per : pieces;
+            for (int c0 = 0; c0 < F; c0 += 32) {
+                const int c = c0 + lane;
+                float acc = 0.f;
+                if (c < F) {
+                    const float* p = a.partial + (size_t)s_first[h] * F + c;
+#pragma unroll 4
+                    for (int k = k0; k < k1; k++) acc = __fadd_rn(acc, __ldg(p + (size_t)k * F));
+                }
+                s_sum[warp][lane] = acc;
+                __syncthreads();
+                if (warp == 0 && c < F) {
+#pragma unroll
+                    for (int q = 1; q < kBlock / 32; q++) acc = __fadd_rn(acc, s_sum[q][lane]);
+                    float* o = a.out + (size_t)s_row[h] * F + c;
+                    *o = finish_value(a, a.accumulate ? __fadd_rn(*o, acc) : acc, (size_t)s_row[h] * F + c, c);
+                }
+                __syncthreads();
+            }
+        }
     }
 }
 
@@ -522,7 +752,7 @@ __global__ void __launch_bounds__(kBlock) hub_fixup_kernel(AggArgs a) {
 // takes at least one ticket (an atomic on one address) to learn that nothing is left, so on a small
 // graph a full grid of some ten thousand warps would spend its time queueing on that counter.
 template <class K>
-static int launch_persistent(K kern, int* blocks_per_sm, const AggArgs& a, cudaStream_t st) {
+static int launch_persistent(K kern, int* blocks_per_sm, const AggArgs& a, cudaStream_t st, int low_grab = 1) {
     if (*blocks_per_sm == 0) {
         int b = 0;
         JG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, kBlock, 0));
@@ -537,6 +767,11 @@ static int launch_persistent(K kern, int* blocks_per_sm, const AggArgs& a, cudaS
     AggArgs b = a;
     const int64_t ids = a.n_out + a.max_items;
     int64_t g = ids / (full * (kBlock / 32) * 24);
+    // A kernel that pays per ticket (the streaming one: look-ups, an open pipeline) takes up to `low_grab` ids at once
+    // as long as that leaves every warp three tickets.
+    int64_t low = ids / (full * (kBlock / 32) * 3);
+    if (low > low_grab) low = low_grab;
+    if (g < low) g = low;
     b.grab = g < 1 ? 1 : (g > kGrab ? kGrab : (int)g);
     const int64_t grabs = (ids + b.grab - 1) / b.grab;
     int64_t blocks = (grabs + kBlock / 32 - 1) / (kBlock / 32);
@@ -547,16 +782,31 @@ static int launch_persistent(K kern, int* blocks_per_sm, const AggArgs& a, cudaS
     return JG_OK;
 }
 
-template <int G, int VPL, int B, int MINB, bool EXACT>
-static int launch_rows(const AggArgs& a, cudaStream_t st) {
-    static int bps[4] = {0, 0, 0, 0};
-    const bool epi = a.bias || a.relu;
-    if (a.f == 4 * G * VPL) {
-        if (epi) return launch_persistent(aggregate_rows_kernel<G, VPL, B, MINB, EXACT, true, true>, &bps[0], a, st);
-        return launch_persistent(aggregate_rows_kernel<G, VPL, B, MINB, EXACT, false, true>, &bps[1], a, st);
+static int epilogue_of(const AggArgs& a) { return a.addend ? kCombine : (a.bias || a.relu) ? kBiasAct : kPlain; }
+
+template <int VPL, int B, int MINB, bool FULL>
+static int launch_rows_as(const AggArgs& a, cudaStream_t st) {
+    static int bps[3] = {0, 0, 0};
+    switch (epilogue_of(a)) {
+        case kPlain: return launch_persistent(aggregate_rows_kernel<VPL, B, MINB, kPlain, FULL>, &bps[0], a, st);
+        case kBiasAct: return launch_persistent(aggregate_rows_kernel<VPL, B, MINB, kBiasAct, FULL>, &bps[1], a, st);
+        default: return launch_persistent(aggregate_rows_kernel<VPL, B, MINB, kCombine, FULL>, &bps[2], a, st);
     }
-    // a narrower 16-byte-aligned width on the same lane layout (the epilogue variant serves both cases)
-    return launch_persistent(aggregate_rows_kernel<G, VPL, B, MINB, EXACT, true, false>, &bps[2], a, st);
+}
+// a narrower 16-byte-aligned width than 128 * VPL runs on the same lane layout
+template <int VPL, int B, int MINB>
+static int launch_rows(const AggArgs& a, cudaStream_t st) {
+    return a.f == 128 * VPL ? launch_rows_as<VPL, B, MINB, true>(a, st) : launch_rows_as<VPL, B, MINB, false>(a, st);
+}
+
+template <int F>
+static int launch_stream(const AggArgs& a, cudaStream_t st) {
+    static int bps[3] = {0, 0, 0};
+    switch (epilogue_of(a)) {
+        case kPlain: return launch_persistent(aggregate_stream_kernel<F, 4, 4, kPlain>, &bps[0], a, st, 4);
+        case kBiasAct: return launch_persistent(aggregate_stream_kernel<F, 4, 4, kBiasAct>, &bps[1], a, st, 4);
+        default: return launch_persistent(aggregate_stream_kernel<F, 4, 4, kCombine>, &bps[2], a, st, 4);
+    }
 }
 
 // Picks the kernel for a feature width: the vector kernel for the 128-bit-aligned widths it is
@@ -564,19 +814,33 @@ static int launch_rows(const AggArgs& a, cudaStream_t st) {
 static int dispatch_aggregate(const AggArgs& a, cudaStream_t st) {
     const int64_t f = a.f;
     const bool vec_ok = (f % 4 == 0) && ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.out) |
-                                          reinterpret_cast<uintptr_t>(a.partial)) % 16 == 0);
-    // widths up to 64 normally put two or four entries of a row side by side in one warp and add the
+                                          reinterpret_cast<uintptr_t>(a.partial) |
+                                          reinterpret_cast<uintptr_t>(a.addend)) % 16 == 0);
+    // widths up to 64 normally put two to four entries of a row side by side in one warp and add the
     // lane groups' partial sums at the end; an ordered sum takes the narrow kernel (F <= 32) or the
     // 128-column layout with idle lanes (F <= 64) instead
-    // (the lane groups' partial sums are added at the end, so these two layouts differ from the sequential
-    // sum by rounding anyway: they use one fused multiply-add per term, half the arithmetic instructions
-    // of the separately rounded form, in a kernel that is bound by instruction issue at these widths)
-    if (vec_ok && f == 32 && !a.ordered) return launch_rows<8, 1, 8, 4, false>(a, st);
-    if (vec_ok && f > 32 && f <= 64 && !a.ordered) return launch_rows<16, 1, 8, 4, false>(a, st);
-    if (vec_ok && f > 32 && f <= 64) return launch_rows<32, 1, 8, 4, true>(a, st);
-    if (vec_ok && f > 64 && f <= 128) return launch_rows<32, 1, 8, 4, true>(a, st);
-    if (vec_ok && f > 128 && f <= 256) return launch_rows<32, 2, 4, 4, true>(a, st);
-    if (vec_ok && f > 256 && f <= 512) return launch_rows<32, 4, 2, 3, true>(a, st);
+    // (with the lane groups' partial sums added at the end the streaming kernel differs from the sequential
+    // sum by rounding anyway: it uses one fused multiply-add per term)
+    // The streaming kernel against the row-by-row one on 8 or 16 lanes, us: 32 columns, 62 M entries 855 -> 780; 64
+    // columns, 132 M 3900 -> 3150; 48 columns, 2.5 M 141 -> 99; 40 columns, 4.9 M 160 -> 152.  Above 64 columns, where a
+    // step is one entry and the sum is in stored order, it was slower (72 columns, 18 M entries: 780 -> 980): unused there.
+    if (vec_ok && !a.ordered) {
+        switch (f) {
+            case 32: return launch_stream<32>(a, st);
+            case 36: return launch_stream<36>(a, st);
+            case 40: return launch_stream<40>(a, st);
+            case 44: return launch_stream<44>(a, st);
+            case 48: return launch_stream<48>(a, st);
+            case 52: return launch_stream<52>(a, st);
+            case 56: return launch_stream<56>(a, st);
+            case 60: return launch_stream<60>(a, st);
+            case 64: return launch_stream<64>(a, st);
+        }
+    }
+    if (vec_ok && f > 32 && f <= 64) return launch_rows<1, 8, 4>(a, st);
+    if (vec_ok && f > 64 && f <= 128) return launch_rows<1, 8, 4>(a, st);
+    if (vec_ok && f > 128 && f <= 256) return launch_rows<2, 4, 4>(a, st);
+    if (vec_ok && f > 256 && f <= 512) return launch_rows<4, 2, 3>(a, st);
     if (f <= 32) {   // narrow rows (any alignment): several rows per warp
         static int nb4 = 0, nb8 = 0, nb16 = 0, nb32 = 0;
         if (f <= 4) return launch_persistent(aggregate_narrow_kernel<4>, &nb4, a, st);
@@ -635,7 +899,7 @@ static int aggregate_impl(float* out, const float* x, const int32_t* idx, const 
                           const float* w, int64_t n_out, int64_t n_in, int64_t f, int64_t nnz,
                           const void* plan, int32_t chunk, void* workspace, size_t workspace_bytes,
                           jg_stream_t stream, int accumulate, const float* bias = nullptr, int relu = 0, int ordered = 0,
-                          int reserve_ctas = 0) {
+                          int reserve_ctas = 0, const float* addend = nullptr, float scale = 1.f, float add_scale = 0.f) {
     JG_CHECK_ARG(n_out >= 0 && n_in >= 0 && f >= 0 && nnz >= 0, JG_EINVAL, "aggregate: negative size");
     if (n_out == 0 || f == 0) return JG_OK;
     JG_CHECK_ARG(out && off, JG_EINVAL, "aggregate: null out/off");
@@ -655,6 +919,7 @@ static int aggregate_impl(float* out, const float* x, const int32_t* idx, const 
     a.relu = relu;
     a.ordered = ordered;
     a.reserve_ctas = reserve_ctas;
+    a.addend = addend; a.scale = scale; a.add_scale = add_scale;
     JG_CHECK_ARG(!bias || f % 4 != 0 || reinterpret_cast<uintptr_t>(bias) % 16 == 0, JG_EINVAL,
                  "aggregate: bias must be 16-byte aligned");
     Carver c(workspace);
@@ -671,7 +936,7 @@ static int aggregate_impl(float* out, const float* x, const int32_t* idx, const 
     int rc = dispatch_aggregate(a, st);
     if (rc != JG_OK) return rc;
     if (plan) {
-        hub_fixup_kernel<<<sm_count() * 2, kBlock, 0, st>>>(a);
+        hub_fixup_kernel<<<sm_count() * 4, kBlock, 0, st>>>(a);
         JG_LAUNCH_CHECK();
     }
     return JG_OK;
@@ -704,6 +969,15 @@ int jg_aggregate_bias_act_f32(float* out, const float* x, const int32_t* idx, co
                               const void* plan, int32_t chunk, void* workspace, size_t workspace_bytes, jg_stream_t stream) {
     return aggregate_impl(out, x, idx, off, w, n_out, n_in, f, nnz, plan, chunk, workspace, workspace_bytes, stream, 0, bias,
                           relu ? 1 : 0);
+}
+
+int jg_aggregate_combine_f32(float* out, const float* x, const int32_t* idx, const int32_t* off, const float* w,
+                             const float* addend, float scale, float add_scale, int64_t n_out, int64_t n_in, int64_t f,
+                             int64_t nnz, const void* plan, int32_t chunk, void* workspace, size_t workspace_bytes,
+                             jg_stream_t stream) {
+    JG_CHECK_ARG(addend || n_out == 0 || f == 0, JG_EINVAL, "aggregate_combine: null addend");
+    return aggregate_impl(out, x, idx, off, w, n_out, n_in, f, nnz, plan, chunk, workspace, workspace_bytes, stream, 0, nullptr,
+                          0, 0, 0, addend, scale, add_scale);
 }
 
 int jg_aggregate_opts_f32(float* out, const float* x, const int32_t* idx, const int32_t* off, const float* w,
@@ -820,7 +1094,7 @@ int jg_aggregate_f32_static(float* out, const float* x, const int32_t* idx, cons
     }
     rc = dispatch_aggregate(a, st);
     if (rc != JG_OK) return rc;
-    hub_fixup_kernel<<<sm_count() * 2, kBlock, 0, st>>>(a);
+    hub_fixup_kernel<<<sm_count() * 4, kBlock, 0, st>>>(a);
     JG_LAUNCH_CHECK();
     return JG_OK;
 }

@@ -106,7 +106,9 @@ class APPNP(torch.nn.Module):
         self.K, self.alpha = K, alpha
 
     def forward(self, x, csc, csr):
-        ah = self.alpha * x                      # alpha * h, formed once
+        if isinstance(self.alpha, (int, float)):
+            return ops.propagate(x, csc, csr, self.K, self.alpha)
+        ah = self.alpha * x                      # a tensor: it may want a gradient of its own
         for _ in range(self.K):
             x = torch.add(ah, ops.aggregateWithWeight(x, csc, csr), alpha=1 - self.alpha)
         return x

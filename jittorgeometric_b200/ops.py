@@ -13,7 +13,7 @@ import torch
 from ._lib import check, lib, ptr, stream_for, workspace
 from .data import CSC, CSR
 
-__all__ = ["aggregateWithWeight", "aggregate_bias_act", "segment_aggregate", "SpmmPlan", "cootocsr", "cootocsc", "gcn_norm_csc_csr",
+__all__ = ["aggregateWithWeight", "aggregate_bias_act", "segment_aggregate", "propagate", "SpmmPlan", "cootocsr", "cootocsc", "gcn_norm_csc_csr",
            "SpmmCsr", "SpmmCoo", "ScatterToEdge", "ScatterToVertex", "EdgeSoftmax", "gat_aggregate",
            "gat_aggregate_supported", "gcn_norm_coo", "linear_tf32", "check_transform_status", "linear_tf32_autograd", "linear_tf32_supported", "matmul_f32", "linear_f32_autograd", "linear_nt", "weight_grad_tf32", "toUndirected", "validate_structure"]
 
@@ -94,7 +94,7 @@ def _plan_of(holder, off, nnz):
 
 
 def segment_aggregate(x, idx, off, w, n_out=None, plan=None, out=None, accumulate=False, bias=None, relu=False,
-                      ordered=False, reserve_ctas=0):
+                      ordered=False, reserve_ctas=0, addend=None, scale=1.0, add_scale=0.0):
     """out[v,:] = sum_{j in [off[v], off[v+1])} w[j] * x[idx[j],:]  (fp32).
 
     The one kernel behind aggregateWithWeight (forward over CSC, backward over
@@ -103,6 +103,8 @@ def segment_aggregate(x, idx, off, w, n_out=None, plan=None, out=None, accumulat
     ``bias`` / ``relu`` fuse the layer epilogue ``act(sum + bias)`` into the store of every row
     (forward only, not together with ``accumulate``).  ``ordered=True`` sums every unsplit row
     strictly in stored order at every width (the default does for widths below 32 and above 64).
+    ``addend`` ([n_out, f]) with ``scale`` and ``add_scale`` stores ``scale * sum + add_scale * addend``
+    (on its own: no bias, ReLU, accumulate, ordered sum or reserved slots with it).
     ``reserve_ctas`` leaves that many CTA slots of the persistent grid free for a kernel on another
     stream (the halo pull of the next exchange)."""
     x = _as_f32(x, "x")
@@ -116,6 +118,12 @@ def segment_aggregate(x, idx, off, w, n_out=None, plan=None, out=None, accumulat
     if w.numel() != nnz:
         raise RuntimeError(f"edge_weight has {w.numel()} entries, indices {nnz}")
     n_in, f = x.shape
+    if addend is not None:
+        if accumulate or bias is not None or relu or ordered or reserve_ctas:
+            raise RuntimeError("segment_aggregate: addend stands on its own")
+        addend = _as_f32(addend, "addend")
+        if addend.shape != (n_out, f):
+            raise RuntimeError(f"addend: expected shape {(n_out, f)}, got {tuple(addend.shape)}")
     if os.environ.get("JG_DEBUG_CHECKS") == "1":
         validate_structure(idx, off, n_in)
     if f > 32 and f % 4 and out is None and not accumulate:
@@ -125,14 +133,20 @@ def segment_aggregate(x, idx, off, w, n_out=None, plan=None, out=None, accumulat
         pad = 4 - f % 4
         xp = torch.nn.functional.pad(x, (0, pad))
         bp = None if bias is None else torch.nn.functional.pad(_as_f32(bias, "bias"), (0, pad))
+        ap = None if addend is None else torch.nn.functional.pad(addend, (0, pad))
         return segment_aggregate(xp, idx, off, w, n_out=n_out, plan=plan, bias=bp, relu=relu, ordered=ordered,
-                                 reserve_ctas=reserve_ctas)[:, :f]
+                                 reserve_ctas=reserve_ctas, addend=ap, scale=scale, add_scale=add_scale)[:, :f]
     if out is None:
         if accumulate:
             raise RuntimeError("accumulate=True needs the tensor to add to (out=)")
         out = torch.empty((n_out, f), dtype=torch.float32, device=x.device)
     chunk = plan.chunk if plan is not None else 0
     ws = workspace(lib().jg_aggregate_workspace_bytes(n_out, nnz, f, chunk), x.device)
+    if addend is not None:
+        check(lib().jg_aggregate_combine_f32(ptr(out), ptr(x), ptr(idx), ptr(off), ptr(w), ptr(addend), float(scale), float(add_scale),
+                                             n_out, n_in, f, nnz, ptr(plan.buf) if plan is not None else None, chunk, ptr(ws),
+                                             ws.numel(), stream_for(x)), "jg_aggregate_combine_f32")
+        return out
     if reserve_ctas:
         b = None if bias is None else _as_f32(bias, "bias")
         if b is not None and b.numel() != f:
@@ -244,6 +258,45 @@ def aggregate_bias_act(x, csc, csr, bias=None, relu=False):
     if bias is None and not relu:
         return aggregateWithWeight(x, csc, csr)
     return _AggregateBiasAct.apply(x, bias, csc, csr, bool(relu))
+
+
+def _entries(container):
+    """Indices, offsets and weights of a CSC or a CSR."""
+    if isinstance(container, CSC):
+        return container.row_indices, container.column_offset, container.edge_weight
+    return container.column_indices, container.row_offset, container.edge_weight
+
+
+class _Propagate(torch.autograd.Function):
+    """``v <- keep * A v + restart * x`` from ``v = x``, ``hops`` times.  The result is a polynomial in A applied to
+    x, so the gradient is the same recursion over the transposed structure, started from the output's gradient:
+    nothing of the forward is kept."""
+
+    @staticmethod
+    def forward(ctx, x, fwd, bwd, hops, restart):
+        ctx.fwd, ctx.bwd, ctx.hops, ctx.restart = fwd, bwd, hops, restart
+        idx, off, w = _entries(fwd)
+        plan = _plan_of(fwd, off, idx.numel())
+        f = x.shape[1]
+        h = _as_f32(x, "x")
+        if f > 32 and f % 4:       # one padded copy for all hops
+            h = torch.nn.functional.pad(h, (0, 4 - f % 4))
+        v = h
+        for _ in range(hops):
+            v = segment_aggregate(v, idx, off, w, plan=plan, addend=h, scale=1 - restart, add_scale=restart)
+        return v if v.shape[1] == f else v[:, :f].contiguous()
+
+    @staticmethod
+    def backward(ctx, grad_output):
+        return _Propagate.apply(grad_output, ctx.bwd, ctx.fwd, ctx.hops, ctx.restart), None, None, None, None
+
+
+def propagate(x, csc, csr, hops, restart):
+    """``hops`` steps of ``v <- (1 - restart) * A v + restart * x`` starting at ``x``
+    (nn/conv/appnp_conv.py:41-52), one kernel per hop in either direction."""
+    if hops <= 0:
+        return x
+    return _Propagate.apply(x, csc, csr, int(hops), float(restart))
 
 
 def _edge_index(edge_index):

@@ -243,3 +243,64 @@ def test_fused_epilogue_autograd(cuda):
         res.append((y.detach(), x.grad, b.grad))
     assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
     assert (res[0][2] - res[1][2]).abs().max().item() <= 1e-4 * res[1][2].abs().max().item()
+
+
+@pytest.mark.parametrize("mode", ["plain", "epilogue", "accumulate", "combine"])
+@pytest.mark.parametrize("f", [5, 32, 36, 40, 44, 48, 64, 72, 130])
+def test_row_lengths_and_epilogues(cuda, oracle, f, mode):
+    """Rows of 0 to 34 entries in every order (runs of empty rows, segments that end on and beside step, batch and window
+    borders), rows one entry above and below the piece length, an infinite value in a row that no entry names.
+    A sum of k terms is off by at most k + 4 roundings (its epilogue's included) of the sum of magnitudes."""
+    rng = np.random.default_rng(f)
+    n_in = 500
+    lens = np.concatenate([np.arange(35), np.zeros(40, int), rng.integers(0, 35, 3000), [63, 64, 65, 200, 127, 128, 129]])
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    idx = rng.integers(1, n_in, off[-1]).astype(np.int32)
+    w = rng.standard_normal(off[-1]).astype(np.float32)
+    x = rng.standard_normal((n_in, f)).astype(np.float32)
+    x[0] = np.inf
+    n = len(lens)
+    other = rng.standard_normal((n, f)).astype(np.float32)
+    bias = rng.standard_normal(f).astype(np.float32)
+    off_t = dev(off)
+    plan = cuda.ops.SpmmPlan(off_t, len(idx), 64)
+    call = lambda **kw: cuda.ops.segment_aggregate(dev(x), dev(idx), off_t, dev(w), plan=plan, **kw)
+    x64 = np.where(np.isfinite(x), x, 0.0)
+    truth, scale = oracle.aggregate_f64(x64.astype(np.float32), idx, off, w)
+    if mode == "plain":
+        got = call()
+    elif mode == "epilogue":
+        got = call(bias=dev(bias), relu=True)
+        truth, scale = np.maximum(truth + bias, 0), scale + np.abs(bias)
+    elif mode == "accumulate":
+        got = call(out=dev(other), accumulate=True)
+        truth, scale = truth + other, scale + np.abs(other)
+    else:
+        got = call(addend=dev(other), scale=0.9, add_scale=0.1)
+        a, b = float(np.float32(0.9)), float(np.float32(0.1))
+        truth, scale = a * truth + b * other, a * scale + b * np.abs(other)
+    assert np.all(np.abs(got.cpu().numpy() - truth) <= (lens[:, None] + 4) * 2.0**-24 * scale + 1e-30)
+
+
+@pytest.mark.parametrize("f", [7, 40, 46])
+def test_propagation_gradient(cuda, f):
+    """The gradient of the hops is the transposed recursion: against float64 autograd, and twice differentiable."""
+    from jittorgeometric_b200 import nn
+    torch.manual_seed(f)
+    n, hops = 300, 4
+    ei = torch.randint(0, n, (2, 4000), device="cuda", dtype=torch.int32)
+    csc, csr = cuda.gcn_norm_csc_csr(ei, None, n)
+    A = torch.zeros((n, n), dtype=torch.float64, device="cuda")
+    dst = torch.repeat_interleave(torch.arange(n, device="cuda"), (csc.column_offset[1:] - csc.column_offset[:-1]).long())
+    A.index_put_((dst, csc.row_indices.long()), csc.edge_weight.double(), accumulate=True)
+    P = torch.eye(n, dtype=torch.float64, device="cuda")
+    for _ in range(hops):
+        P = 0.9 * (A @ P) + 0.1 * torch.eye(n, dtype=torch.float64, device="cuda")
+    x = torch.randn((n, f), device="cuda", requires_grad=True)
+    g = torch.randn((n, f), device="cuda", requires_grad=True)
+    y = nn.APPNP(hops, 0.1)(x, csc, csr)
+    assert y.is_contiguous()
+    gx, = torch.autograd.grad(y, x, g, create_graph=True)
+    gg, = torch.autograd.grad(gx, g, x)          # the product is linear in g: its derivative along x is P x
+    for have, want in ((y, P @ x.double()), (gx, P.t() @ g.double()), (gg, P @ x.double())):
+        assert (have.double() - want).abs().max().item() <= 1e-5 * want.abs().max().item()
