@@ -54,6 +54,7 @@ SIGNATURES = {
     "jg_gather_rows_f32": (ctypes.c_int, [vp, vp, vp, i64, i64, i32, vp]),
     "jg_convert_workspace_bytes": (sz, [i64, i64]),
     "jg_coo_to_compressed": (ctypes.c_int, [vp, vp, i64, i64, ctypes.c_int, ctypes.c_int, vp, vp, vp, vp, sz, vp]),
+    "jg_group_edges": (ctypes.c_int, [vp, i64, i64, vp, vp, vp, vp, sz, vp]),
     "jg_gcn_norm_compressed": (ctypes.c_int, [vp, vp, i64, i64, f32, ctypes.c_int, ctypes.c_int, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp]),
     "jg_gcn_norm_coo_workspace_bytes": (sz, [i64, i64]),
     "jg_gcn_norm_coo": (ctypes.c_int, [vp, vp, i64, i64, f32, ctypes.c_int, vp, vp, vp, vp, vp, sz, vp]),

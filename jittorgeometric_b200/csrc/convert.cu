@@ -142,14 +142,17 @@ struct Raw {
 
 __device__ __forceinline__ int64_t list_count(const SortSrc& s) { return s.dcount ? (int64_t)*s.dcount : s.count; }
 
+// MODE (0, 1, 2 as in SortSrc) is a template parameter: with the tests of the other modes compiled in, the first pass of a
+// COO list carried their registers and branches (285 M entries: one more of them cost 0.75 ms a pass).
+template <int MODE>
 __device__ __forceinline__ Raw load_raw(const SortSrc& s, int64_t p, int64_t count) {
     Raw r;
     r.a = 0; r.b = 0; r.w = 1.f;
     if (p >= count) return r;
-    if (s.mode == 0) {
+    if (MODE == 0) {
         r.a = s.key[p]; r.b = s.idx[p];
         if (s.w) r.w = s.w[p];
-    } else if (s.mode == 2) {
+    } else if (MODE == 2) {
         // mirrored list: position 2i is edge i as given, 2i + 1 the same edge reversed
         const int64_t i = p >> 1;
         r.a = s.coo_src[i]; r.b = s.coo_dst[i];
@@ -165,22 +168,22 @@ __device__ __forceinline__ Raw load_raw(const SortSrc& s, int64_t p, int64_t cou
     return r;
 }
 
+template <int MODE>
 __device__ __forceinline__ Elem finish_elem(const SortSrc& s, int64_t p, int64_t count, const Raw& r) {
     Elem e;
     e.valid = p < count;
     e.key = 0; e.idx = 0; e.w = r.w;
     if (!e.valid) { e.w = 0.f; return e; }
-    if (s.mode == 0) {
+    if (MODE == 0) {
         e.key = r.a; e.idx = r.b;
-    } else if (s.mode == 2) {
+    } else if (MODE == 2) {
         e.key = (p & 1) ? r.b : r.a;
         e.idx = (p & 1) ? r.a : r.b;
-    } else if (p < s.e0) {
+    } else {
+        // an appended loop has a == b, so the swap does not matter to it
         e.key = s.by == 0 ? r.a : r.b;
         e.idx = s.by == 0 ? r.b : r.a;
-        if (s.drop_loops && r.a == r.b) e.valid = false;
-    } else {
-        e.key = r.a; e.idx = r.a;
+        if (s.drop_loops && r.a == r.b && p < s.e0) e.valid = false;
     }
     return e;
 }
@@ -190,10 +193,8 @@ __device__ __forceinline__ int digit_of(const Elem& e, int shift, int from_idx) 
     return ((from_idx ? e.idx : e.key) >> shift) & (kRadix - 1);
 }
 
-// SORTED: the source is a sorted buffer (mode 0); a separate instantiation, so that the register needs of the
-// first pass's element loader do not lower the occupancy of the other passes.
 constexpr int kHistThreads = kSortThreads;
-template <bool SORTED, int ITEMS>
+template <int MODE, int ITEMS>
 __global__ void __launch_bounds__(kHistThreads) sort_hist_kernel(SortSrc s, int shift, int from_idx, int* __restrict__ matrix) {
     __shared__ int s_hist[kRadix];
     constexpr int kSortTile = kSortThreads * ITEMS;
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(kHistThreads) sort_hist_kernel(SortSrc s, int 
     __syncthreads();
     const int64_t base = (int64_t)blockIdx.x * kSortTile;
     const int64_t count = list_count(s);
-    if (SORTED) {
+    if (MODE == 0) {
         // sorted-buffer passes: only the array the digit comes from is read (half the bytes of a full element)
         const int32_t* from = from_idx ? s.idx : s.key;
         if (base + kSortTile <= count && reinterpret_cast<uintptr_t>(from) % 16 == 0) {
@@ -229,10 +230,10 @@ __global__ void __launch_bounds__(kHistThreads) sort_hist_kernel(SortSrc s, int 
         for (int i0 = 0; i0 < kRounds; i0 += kBatch) {
             Raw raw[kBatch];
 #pragma unroll
-            for (int i = 0; i < kBatch; i++) raw[i] = load_raw(s, base + (int64_t)(i0 + i) * kHistThreads + threadIdx.x, count);   // all loads in flight
+            for (int i = 0; i < kBatch; i++) raw[i] = load_raw<MODE>(s, base + (int64_t)(i0 + i) * kHistThreads + threadIdx.x, count);   // all loads in flight
 #pragma unroll
             for (int i = 0; i < kBatch; i++) {
-                const Elem e = finish_elem(s, base + (int64_t)(i0 + i) * kHistThreads + threadIdx.x, count, raw[i]);
+                const Elem e = finish_elem<MODE>(s, base + (int64_t)(i0 + i) * kHistThreads + threadIdx.x, count, raw[i]);
                 if (e.valid) atomicAdd(&s_hist[digit_of(e, shift, from_idx)], 1);
             }
         }
@@ -260,10 +261,10 @@ __global__ void __launch_bounds__(kHistThreads) sort_hist_both_kernel(SortSrc s,
     for (int i0 = 0; i0 < kRounds; i0 += kBatch) {
         Raw raw[kBatch];
 #pragma unroll
-        for (int i = 0; i < kBatch; i++) raw[i] = load_raw(s, base + (int64_t)(i0 + i) * kHistThreads + threadIdx.x, count);
+        for (int i = 0; i < kBatch; i++) raw[i] = load_raw<1>(s, base + (int64_t)(i0 + i) * kHistThreads + threadIdx.x, count);
 #pragma unroll
         for (int i = 0; i < kBatch; i++) {
-            const Elem e = finish_elem(s, base + (int64_t)(i0 + i) * kHistThreads + threadIdx.x, count, raw[i]);
+            const Elem e = finish_elem<1>(s, base + (int64_t)(i0 + i) * kHistThreads + threadIdx.x, count, raw[i]);
             if (e.valid) {
                 const int src = s.by == 0 ? e.key : e.idx, dst = s.by == 0 ? e.idx : e.key;
                 atomicAdd(&s_hist[0][dst & (kRadix - 1)], 1);
@@ -286,8 +287,7 @@ struct SortDst {
 // order of the source list because warp w reads one contiguous range of 32 * kSortItems entries.
 // HAS_W = false: every weight is 1 (no input weights), so the sort moves (key, index) pairs only and
 // the caller writes the weights afterwards; a third less traffic per pass.
-// SORTED: the source is a buffer (mode 0); the first pass's element loader is an instantiation of its own.
-template <bool HAS_W, bool SORTED, int ITEMS>
+template <bool HAS_W, int MODE, int ITEMS>
 __global__ void __launch_bounds__(kSortThreads, ITEMS == kItemsMany ? 3 : 4) sort_scatter_kernel(SortSrc s, SortDst d, int shift, int from_idx,
                                                                                                 const int* __restrict__ matrix) {
     constexpr int kSortItems = ITEMS;
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kSortThreads, ITEMS == kItemsMany ? 3 : 4) sor
     float wt[HAS_W ? kSortItems : 1];
     unsigned valid = 0;
     // every load of the tile first (independent, all in flight), the ranking rounds after them
-    if (SORTED) {
+    if (MODE == 0) {
 #pragma unroll
         for (int r = 0; r < kSortItems; r++) {
             const int64_t p = wbase + r * 32 + lane;
@@ -322,10 +322,10 @@ __global__ void __launch_bounds__(kSortThreads, ITEMS == kItemsMany ? 3 : 4) sor
     } else {
         Raw raw[kSortItems];
 #pragma unroll
-        for (int r = 0; r < kSortItems; r++) raw[r] = load_raw(s, wbase + r * 32 + lane, count);
+        for (int r = 0; r < kSortItems; r++) raw[r] = load_raw<MODE>(s, wbase + r * 32 + lane, count);
 #pragma unroll
         for (int r = 0; r < kSortItems; r++) {
-            const Elem e = finish_elem(s, wbase + r * 32 + lane, count, raw[r]);
+            const Elem e = finish_elem<MODE>(s, wbase + r * 32 + lane, count, raw[r]);
             key[r] = e.key; idx[r] = e.idx;
             if (HAS_W) wt[r] = e.w;
             valid |= e.valid ? 1u << r : 0u;
@@ -413,17 +413,20 @@ constexpr size_t scatter_smem(bool has_w, int items) {
 }
 
 typedef void (*ScatterFn)(SortSrc, SortDst, int, int, const int*);
-static ScatterFn scatter_fn(bool has_w, bool sorted, int items) {
-    if (has_w) return sorted ? sort_scatter_kernel<true, true, kItemsFew> : sort_scatter_kernel<true, false, kItemsFew>;
-    if (items == kItemsFew) return sorted ? sort_scatter_kernel<false, true, kItemsFew> : sort_scatter_kernel<false, false, kItemsFew>;
-    return sorted ? sort_scatter_kernel<false, true, kItemsMany> : sort_scatter_kernel<false, false, kItemsMany>;
+typedef void (*HistFn)(SortSrc, int, int, int*);
+// The instantiations: a list with weights takes kItemsFew, a mirrored list (mode 2) always has weights.
+static ScatterFn scatter_fn(bool has_w, int mode, int items) {
+    if (has_w)
+        return mode == 0 ? sort_scatter_kernel<true, 0, kItemsFew> : mode == 1 ? sort_scatter_kernel<true, 1, kItemsFew>
+                                                                               : sort_scatter_kernel<true, 2, kItemsFew>;
+    if (mode == 2) return nullptr;
+    if (items == kItemsFew) return mode == 0 ? sort_scatter_kernel<false, 0, kItemsFew> : sort_scatter_kernel<false, 1, kItemsFew>;
+    return mode == 0 ? sort_scatter_kernel<false, 0, kItemsMany> : sort_scatter_kernel<false, 1, kItemsMany>;
 }
-
-static void launch_hist(const SortSrc& src, int shift, int from_idx, int* matrix, int64_t tiles, int items, cudaStream_t st) {
-    const bool sorted = src.mode == 0;
-    auto kern = items == kItemsFew ? (sorted ? sort_hist_kernel<true, kItemsFew> : sort_hist_kernel<false, kItemsFew>)
-                                   : (sorted ? sort_hist_kernel<true, kItemsMany> : sort_hist_kernel<false, kItemsMany>);
-    kern<<<(unsigned)tiles, kHistThreads, 0, st>>>(src, shift, from_idx, matrix);
+static HistFn hist_fn(int mode, int items) {
+    if (mode == 2) return sort_hist_kernel<2, kItemsFew>;
+    if (items == kItemsFew) return mode == 0 ? sort_hist_kernel<0, kItemsFew> : sort_hist_kernel<1, kItemsFew>;
+    return mode == 0 ? sort_hist_kernel<0, kItemsMany> : sort_hist_kernel<1, kItemsMany>;
 }
 
 // ------------------------------------------------------------------------------- small kernels
@@ -735,6 +738,11 @@ __global__ void split_offsets_kernel(const int32_t* __restrict__ off, const int*
     }
 }
 
+__global__ void iota_kernel(int* p, int64_t n) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) p[i] = (int)i;
+}
+
 __global__ void fill_int_kernel(int* p, int v, int64_t n) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) p[i] = v;
@@ -796,17 +804,20 @@ static int radix_sort(SortSrc first, int64_t n, int canonical, const unsigned lo
     int dev = 0;
     JG_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        for (int v = 0; v < 6; v++) {
-            const bool has_w = v >= 4, sorted = v & 1;
-            const int items = v >= 2 && v < 4 ? kItemsMany : kItemsFew;
-            JG_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(scatter_fn(has_w, sorted, items)),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem(has_w, items)));
+        for (int v = 0; v < 12; v++) {
+            const bool has_w = v >= 6;
+            const int mode = v % 3, items = v % 6 >= 3 ? kItemsMany : kItemsFew;
+            ScatterFn fn = has_w && items == kItemsMany ? nullptr : scatter_fn(has_w, mode, items);
+            if (fn)
+                JG_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)scatter_smem(has_w, items)));
         }
         attr_set[dev] = true;
     }
     const int bits = bits_for(n);
     const int key_passes = (bits + 7) / 8;
     const int total_passes = canonical ? 2 * key_passes : key_passes;
+    JG_CHECK_ARG(first.mode != 2 || carry_w, JG_EINVAL, "radix_sort: a mirrored list carries weights");
     const int items = sort_items(first.count, carry_w);
     const int64_t tiles = sort_tiles(first.count, items);  // upper bound for every pass
     SortSrc src = first;
@@ -820,7 +831,7 @@ static int radix_sort(SortSrc first, int64_t n, int canonical, const unsigned lo
         if (p == 0 && counted) {
             matrix = counted;
         } else {
-            launch_hist(src, shift, from_idx, matrix, tiles, items, st);
+            hist_fn(src.mode, items)<<<(unsigned)tiles, kHistThreads, 0, st>>>(src, shift, from_idx, matrix);
             JG_LAUNCH_CHECK();
         }
         if (tiles <= kChunkTiles) {
@@ -840,7 +851,7 @@ static int radix_sort(SortSrc first, int64_t n, int canonical, const unsigned lo
         dst.key = ws.key[cur];
         dst.idx = last ? out_idx : ws.idx[cur];
         dst.w = carry_w ? (last ? out_w : ws.w[cur]) : nullptr;
-        scatter_fn(carry_w, src.mode == 0, items)<<<(unsigned)tiles, kSortThreads, scatter_smem(carry_w, items), st>>>(src, dst, shift, from_idx, matrix);
+        scatter_fn(carry_w, src.mode, items)<<<(unsigned)tiles, kSortThreads, scatter_smem(carry_w, items), st>>>(src, dst, shift, from_idx, matrix);
         JG_LAUNCH_CHECK();
         *sorted_key = dst.key;
         SortSrc nxt = {};
@@ -893,6 +904,39 @@ int jg_coo_to_compressed(const int32_t* edge_index, const float* w, int64_t n_ed
     if (rc != JG_OK) return rc;
     if (!carry_w && n_edges > 0) {   // no input weights: every output weight is 1.0f
         fill_int_kernel<<<blocks_for(n_edges, 256), 256, 0, st>>>(reinterpret_cast<int*>(out_w), 0x3f800000, n_edges);
+        JG_LAUNCH_CHECK();
+    }
+    offsets_from_sorted_keys<<<offset_blocks(n_edges), kOffThreads, 0, st>>>(skey, n_edges, nullptr, n_nodes, out_off);
+    JG_LAUNCH_CHECK();
+    return JG_OK;
+}
+
+int jg_group_edges(const int32_t* node, int64_t n_edges, int64_t n_nodes, int32_t* out_edge, int32_t* out_off, float* out_ones,
+                   void* workspace, size_t workspace_bytes, jg_stream_t stream) {
+    JG_CHECK_ARG(n_edges >= 0 && n_nodes >= 0, JG_EINVAL, "group_edges: negative size");
+    JG_CHECK_ARG(out_off && (n_edges == 0 || (node && out_edge)), JG_EINVAL, "group_edges: null array");
+    JG_CHECK_ARG(n_edges <= INT32_MAX - 1 && n_nodes < INT32_MAX, JG_ESHAPE, "group_edges: sizes beyond int32");
+    JG_CHECK_ARG(workspace && workspace_bytes >= jg_convert_workspace_bytes(n_edges, n_nodes), JG_EWORKSPACE,
+                 "group_edges: workspace %zu < %zu", workspace_bytes, jg_convert_workspace_bytes(n_edges, n_nodes));
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    ConvertWs ws = carve_convert(workspace, n_edges + n_nodes, n_nodes);
+    SortSrc first = {};
+    // the second buffer's indices are written only after the first pass has read the positions from there
+    first.mode = 1;
+    first.coo_src = node;
+    first.coo_dst = ws.idx[1];
+    if (n_edges > 0) {
+        iota_kernel<<<blocks_for(n_edges, 256), 256, 0, st>>>(ws.idx[1], n_edges);
+        JG_LAUNCH_CHECK();
+    }
+    first.e0 = n_edges;
+    first.by = 0;
+    first.count = n_edges;
+    int32_t* skey = nullptr;
+    int rc = radix_sort(first, n_nodes, 0, nullptr, ws, out_edge, nullptr, &skey, st, false);
+    if (rc != JG_OK) return rc;
+    if (out_ones && n_edges > 0) {
+        fill_int_kernel<<<blocks_for(n_edges, 256), 256, 0, st>>>(reinterpret_cast<int*>(out_ones), 0x3f800000, n_edges);
         JG_LAUNCH_CHECK();
     }
     offsets_from_sorted_keys<<<offset_blocks(n_edges), kOffThreads, 0, st>>>(skey, n_edges, nullptr, n_nodes, out_off);

@@ -59,6 +59,8 @@ static PlanView plan_view(void* plan, int64_t nnz, int32_t chunk, size_t* bytes)
     return v;
 }
 
+__global__ void plan_header_kernel(PlanHeader* hdr, PlanHeader h) { *hdr = h; }
+
 __global__ void plan_build_kernel(const int32_t* __restrict__ off, int64_t n, PlanView p, int32_t chunk) {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n;
          v += (int64_t)gridDim.x * blockDim.x) {
@@ -876,8 +878,10 @@ int jg_spmm_plan_build(const int32_t* off, int64_t n_out, int64_t nnz, int32_t c
     PlanView v = plan_view(plan, nnz, chunk, &need);
     JG_CHECK_ARG(plan_bytes >= need, JG_EWORKSPACE, "plan_build: plan buffer %zu < %zu", plan_bytes, need);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    PlanHeader h = {0, 0, chunk, (int32_t)plan_max_hubs(nnz, chunk), (int32_t)plan_max_items(nnz, chunk), {0, 0, 0}};
-    JG_CUDA(cudaMemcpyAsync(v.hdr, &h, sizeof(h), cudaMemcpyHostToDevice, st));
+    // written by a kernel from its arguments: a copy from this frame would be read at replay under stream capture
+    plan_header_kernel<<<1, 1, 0, st>>>(v.hdr, PlanHeader{0, 0, chunk, (int32_t)plan_max_hubs(nnz, chunk),
+                                                          (int32_t)plan_max_items(nnz, chunk), {0, 0, 0}});
+    JG_LAUNCH_CHECK();
     if (n_out > 0) {
         int grid = (int)((n_out + 255) / 256);
         if (grid > sm_count() * 16) grid = sm_count() * 16;

@@ -241,6 +241,22 @@ def test_scatter_to_edge_backward_by_source(cuda, c, edges):
     assert np.all(np.abs(host(x.grad) - want) <= terms * 2.0**-24 * mag)
 
 
+@pytest.mark.parametrize("edges", [0, 1, 2048, 2049, 270001])
+@pytest.mark.parametrize("c", [24, 30, 32, 64, 128])
+def test_sum_by_source_over_grouped_edges(cuda, c, edges):
+    """The path of large edge tensors, called at its tile borders: every edge's row reaches its source once.  The error
+    bound of a sum of k terms in any order, as above."""
+    n, rng = 300, np.random.default_rng(c + edges)
+    idx = np.minimum((rng.random(edges) ** 3 * n).astype(np.int32), n - 1)
+    m = rng.standard_normal((edges, c)).astype(np.float32)
+    got = host(cuda.ops._sum_by_source(dev(m), dev(idx), n))
+    order = np.argsort(idx, kind="stable")
+    starts = np.concatenate([[0], np.cumsum(np.bincount(idx, minlength=n))])
+    for v in range(n):
+        rows = m[order[starts[v]:starts[v + 1]]].astype(np.float64)
+        assert np.all(np.abs(got[v] - rows.sum(0)) <= (len(rows) + 1) * 2.0**-24 * np.abs(rows).sum(0))
+
+
 def attention_truth(h, a_src, a_dst, idx, off, slope=0.2):
     """Differentiable float64 restatement of the edge phase with plain tensor operations."""
     n, heads, dim = h.shape[0], a_src.shape[0], a_src.shape[1]
