@@ -687,11 +687,12 @@ __global__ void __launch_bounds__(kBlock) aggregate_narrow_kernel(AggArgs a) {
 // counts and first slots are read side by side, then hubs of up to kFewPieces pieces are summed with one thread per
 // (hub, column), all pieces in flight, and the others one by one by the whole block, eight warps each adding an eighth
 // of the pieces in order and the eighths in order.  With one thread per (hub, column) whatever the pieces, the
-// longest hub's chain of loads was the kernel: 17 us beside a 160 us aggregation of 4.9 M entries (70 pieces).
+// longest hub's chain of loads was the kernel: 17 us beside a 160 us aggregation of 4.9 M entries (70 pieces), 8 us so;
+// 128 columns at a time (16 bytes a lane) where the width allows: 256 columns, 126 M entries 207 -> 94 us.
 constexpr int kFewPieces = 8;
 __global__ void __launch_bounds__(kBlock) hub_fixup_kernel(AggArgs a) {
     __shared__ int s_row[kBlock], s_first[kBlock], s_pieces[kBlock];
-    __shared__ float s_sum[kBlock / 32][32];
+    __shared__ float4 s_sum[kBlock / 32][32];
     const int n_hubs = a.hdr->n_hubs;
     const int chunk = a.hdr->chunk;
     const int F = (int)a.f;
@@ -728,21 +729,35 @@ __global__ void __launch_bounds__(kBlock) hub_fixup_kernel(AggArgs a) {
             if (pieces <= kFewPieces) continue;
             const int per = (pieces + kBlock / 32 - 1) / (kBlock / 32);
             const int k0 = warp * per, k1 = k0 + per < pieces ? k0 + per : pieces;
-            for (int c0 = 0; c0 < F; c0 += 32) {
-                const int c = c0 + lane;
-                float acc = 0.f;
+            const int V = F % 4 == 0 ? 4 : 1;      // partial rows start on 16-byte borders then
+            for (int c0 = 0; c0 < F; c0 += 32 * V) {
+                const int c = c0 + lane * V;
+                float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (c < F) {
                     const float* p = a.partial + (size_t)s_first[h] * F + c;
+                    if (V == 4) {
 #pragma unroll 4
-                    for (int k = k0; k < k1; k++) acc = __fadd_rn(acc, __ldg(p + (size_t)k * F));
+                        for (int k = k0; k < k1; k++) {
+                            const float4 v = __ldg(reinterpret_cast<const float4*>(p + (size_t)k * F));
+                            acc.x = __fadd_rn(acc.x, v.x); acc.y = __fadd_rn(acc.y, v.y);
+                            acc.z = __fadd_rn(acc.z, v.z); acc.w = __fadd_rn(acc.w, v.w);
+                        }
+                    } else {
+#pragma unroll 4
+                        for (int k = k0; k < k1; k++) acc.x = __fadd_rn(acc.x, __ldg(p + (size_t)k * F));
+                    }
                 }
                 s_sum[warp][lane] = acc;
                 __syncthreads();
-                if (warp == 0 && c < F) {
+                // one thread per column of the slab: the eighths in order
+                const int col = c0 + (int)threadIdx.x;
+                if ((int)threadIdx.x < 32 * V && col < F) {
+                    const int l = threadIdx.x / V, q = threadIdx.x % V;
+                    float sum = reinterpret_cast<const float*>(&s_sum[0][l])[q];
 #pragma unroll
-                    for (int q = 1; q < kBlock / 32; q++) acc = __fadd_rn(acc, s_sum[q][lane]);
-                    float* o = a.out + (size_t)s_row[h] * F + c;
-                    *o = finish_value(a, a.accumulate ? __fadd_rn(*o, acc) : acc, (size_t)s_row[h] * F + c, c);
+                    for (int g = 1; g < kBlock / 32; g++) sum = __fadd_rn(sum, reinterpret_cast<const float*>(&s_sum[g][l])[q]);
+                    float* o = a.out + (size_t)s_row[h] * F + col;
+                    *o = finish_value(a, a.accumulate ? __fadd_rn(*o, sum) : sum, (size_t)s_row[h] * F + col, col);
                 }
                 __syncthreads();
             }
