@@ -597,7 +597,8 @@ __global__ void __launch_bounds__(kBlock) aggregate_any_kernel(AggArgs a) {
 // each and hand them round with width-G shuffles; lane c gathers column c of every source row.
 // All groups run the trip count of the longest of their segments, with predicates, so the shuffles
 // stay convergent.  The last layer of a GCN (a handful of classes) is this shape.
-template <int G>
+// EPI: an epilogue is asked for (with its tests in the plain form, 14 columns and 10 M entries took 2 % longer).
+template <int G, bool EPI>
 __global__ void __launch_bounds__(kBlock) aggregate_narrow_kernel(AggArgs a) {
     constexpr int R = 32 / G;          // work ids per warp step
     constexpr int ROUNDS = 4;          // steps per ticket
@@ -675,7 +676,7 @@ __global__ void __launch_bounds__(kBlock) aggregate_narrow_kernel(AggArgs a) {
                 float v = acc;
                 if (final_row) {
                     if (a.accumulate) v = __fadd_rn(dst[c], v);
-                    v = finish_value(a, v, (size_t)(dst - a.out) + c, c);
+                    if (EPI) v = finish_value(a, v, (size_t)(dst - a.out) + c, c);
                 }
                 dst[c] = v;
             }
@@ -709,8 +710,9 @@ __global__ void __launch_bounds__(kBlock) hub_fixup_kernel(AggArgs a) {
             s_pieces[threadIdx.x] = (a.off[row + 1] - a.off[row] + chunk - 1) / chunk;
         }
         __syncthreads();
-        for (int t = threadIdx.x; t < cnt * F; t += kBlock) {
-            const int h = t / F, c = t - h * F;
+        const int64_t values = (int64_t)cnt * F;
+        for (int64_t t = threadIdx.x; t < values; t += kBlock) {
+            const int h = values < INT32_MAX ? (int)t / F : (int)(t / F), c = (int)(t - (int64_t)h * F);
             const int pieces = s_pieces[h];
             if (pieces > kFewPieces) continue;
             const float* p = a.partial + (size_t)s_first[h] * F + c;
@@ -826,6 +828,13 @@ static int launch_stream(const AggArgs& a, cudaStream_t st) {
     }
 }
 
+template <int G>
+static int launch_narrow(const AggArgs& a, cudaStream_t st) {
+    static int bps[2] = {0, 0};
+    if (epilogue_of(a) != kPlain) return launch_persistent(aggregate_narrow_kernel<G, true>, &bps[0], a, st);
+    return launch_persistent(aggregate_narrow_kernel<G, false>, &bps[1], a, st);
+}
+
 // Picks the kernel for a feature width: the vector kernel for the 128-bit-aligned widths it is
 // specialised for, the column-strided kernel for everything else.
 static int dispatch_aggregate(const AggArgs& a, cudaStream_t st) {
@@ -859,11 +868,10 @@ static int dispatch_aggregate(const AggArgs& a, cudaStream_t st) {
     if (vec_ok && f > 128 && f <= 256) return launch_rows<2, 4, 4>(a, st);
     if (vec_ok && f > 256 && f <= 512) return launch_rows<4, 2, 3>(a, st);
     if (f <= 32) {   // narrow rows (any alignment): several rows per warp
-        static int nb4 = 0, nb8 = 0, nb16 = 0, nb32 = 0;
-        if (f <= 4) return launch_persistent(aggregate_narrow_kernel<4>, &nb4, a, st);
-        if (f <= 8) return launch_persistent(aggregate_narrow_kernel<8>, &nb8, a, st);
-        if (f <= 16) return launch_persistent(aggregate_narrow_kernel<16>, &nb16, a, st);
-        return launch_persistent(aggregate_narrow_kernel<32>, &nb32, a, st);
+        if (f <= 4) return launch_narrow<4>(a, st);
+        if (f <= 8) return launch_narrow<8>(a, st);
+        if (f <= 16) return launch_narrow<16>(a, st);
+        return launch_narrow<32>(a, st);
     }
     static int any2 = 0, any4 = 0, any8 = 0;
     if (f <= 64) return launch_persistent(aggregate_any_kernel<2>, &any2, a, st);
