@@ -339,14 +339,17 @@ __global__ void __launch_bounds__(kBlock, MINB) aggregate_stream_kernel(AggArgs 
     const char* xb = reinterpret_cast<const char*>(a.x) + fl * 16;
     const int64_t n_items = a.hdr ? a.hdr->n_items : 0;
     const int chunk = a.hdr ? a.hdr->chunk : 0x7fffffff;
-    const int64_t total = n_items + a.n_out;
     const int grab = a.grab;
+    // a piece of a hub is a ticket of its own (with four of them in one warp a small graph's tail was longer than its
+    // work: 50 k rows, 1.3 M entries, 36 columns, both directions 0.20 ms against 0.12 of the row kernel on 16 lanes), rows come `grab` at a time
+    const int64_t tickets = n_items + (a.n_out + grab - 1) / grab;
+    auto first_id = [&](int64_t ticket) { return ticket < n_items ? ticket : n_items + (ticket - n_items) * grab; };
 
     // lane i's segment of the ticket: first entry and length (-1: none, a hub row is walked as pieces)
-    auto load_segments = [&](int64_t base, int& s, int& len) {
+    auto load_segments = [&](int64_t ticket, int& s, int& len) {
         s = 0; len = -1;
-        const int64_t id = base + lane;
-        if (lane < grab && id < total) {
+        const int64_t id = first_id(ticket) + lane;
+        if (lane < (ticket < n_items ? 1 : grab) && id < n_items + a.n_out) {
             if (id < n_items) {
                 const int h = a.item_hub[id], k = a.item_k[id];
                 const int row = a.hub_row[h];
@@ -360,18 +363,19 @@ __global__ void __launch_bounds__(kBlock, MINB) aggregate_stream_kernel(AggArgs 
             }
         }
     };
-    auto take = [&]() -> unsigned long long { return lane == 0 ? atomicAdd(a.ticket, (unsigned long long)grab) : 0ull; };
+    auto take = [&]() -> unsigned long long { return lane == 0 ? atomicAdd(a.ticket, 1ull) : 0ull; };
 
-    int64_t base = (int64_t)__shfl_sync(kFull, take(), 0);
-    if (base >= total) return;
+    int64_t ticket = (int64_t)__shfl_sync(kFull, take(), 0);
+    if (ticket >= tickets) return;
     int seg_s, seg_len;
-    load_segments(base, seg_s, seg_len);
+    load_segments(ticket, seg_s, seg_len);
     unsigned long long coming = take();
     for (;;) {
-        const int64_t next_base = (int64_t)__shfl_sync(kFull, coming, 0);
+        const int64_t base = first_id(ticket);
+        const int64_t next_ticket = (int64_t)__shfl_sync(kFull, coming, 0);
         int nxt_s, nxt_len;
-        load_segments(next_base, nxt_s, nxt_len);
-        if (next_base < total) coming = take();
+        load_segments(next_ticket, nxt_s, nxt_len);
+        if (next_ticket < tickets) coming = take();
 
         const int padded = seg_len > 0 ? (seg_len + EPS - 1) / EPS * EPS : 0;
         int incl = padded;
@@ -486,8 +490,8 @@ __global__ void __launch_bounds__(kBlock, MINB) aggregate_stream_kernel(AggArgs 
                 consume(v1, bi + 1);
             }
         }
-        if (next_base >= total) break;
-        base = next_base;
+        if (next_ticket >= tickets) break;
+        ticket = next_ticket;
         seg_s = nxt_s; seg_len = nxt_len;
     }
 }
@@ -787,12 +791,13 @@ static int launch_persistent(K kern, int* blocks_per_sm, const AggArgs& a, cudaS
     const int64_t ids = a.n_out + a.max_items;
     int64_t g = ids / (full * (kBlock / 32) * 24);
     // A kernel that pays per ticket (the streaming one: look-ups, an open pipeline) takes up to `low_grab` ids at once
-    // as long as that leaves every warp three tickets.
-    int64_t low = ids / (full * (kBlock / 32) * 3);
+    // as long as that leaves every warp six tickets.
+    int64_t low = ids / (full * (kBlock / 32) * 6);
     if (low > low_grab) low = low_grab;
     if (g < low) g = low;
     b.grab = g < 1 ? 1 : (g > kGrab ? kGrab : (int)g);
-    const int64_t grabs = (ids + b.grab - 1) / b.grab;
+    const int64_t grabs = low_grab > 1 ? a.max_items + (a.n_out + b.grab - 1) / b.grab     // a piece is a ticket of its own there
+                                       : (ids + b.grab - 1) / b.grab;
     int64_t blocks = (grabs + kBlock / 32 - 1) / (kBlock / 32);
     if (blocks > full) blocks = full;
     if (blocks < 1) blocks = 1;
