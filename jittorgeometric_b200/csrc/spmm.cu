@@ -704,6 +704,8 @@ __global__ void __launch_bounds__(kBlock) hub_fixup_kernel(AggArgs a) {
     const int lane = lane_id(), warp = threadIdx.x / 32;
     int per_block = (n_hubs + (int)gridDim.x - 1) / (int)gridDim.x;
     if (per_block > kBlock) per_block = kBlock;
+    // 16 bytes a lane where every partial row starts on a 16-byte border; a caller's workspace need not
+    const int V = F % 4 == 0 && reinterpret_cast<uintptr_t>(a.partial) % 16 == 0 ? 4 : 1;
     for (int64_t h0 = (int64_t)blockIdx.x * per_block; h0 < n_hubs; h0 += (int64_t)gridDim.x * per_block) {
         const int cnt = n_hubs - h0 < per_block ? (int)(n_hubs - h0) : per_block;
         __syncthreads();
@@ -735,7 +737,6 @@ __global__ void __launch_bounds__(kBlock) hub_fixup_kernel(AggArgs a) {
             if (pieces <= kFewPieces) continue;
             const int per = (pieces + kBlock / 32 - 1) / (kBlock / 32);
             const int k0 = warp * per, k1 = k0 + per < pieces ? k0 + per : pieces;
-            const int V = F % 4 == 0 ? 4 : 1;      // partial rows start on 16-byte borders then
             for (int c0 = 0; c0 < F; c0 += 32 * V) {
                 const int c = c0 + lane * V;
                 float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);

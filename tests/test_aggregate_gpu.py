@@ -304,3 +304,28 @@ def test_propagation_gradient(cuda, f):
     gg, = torch.autograd.grad(gx, g, x)          # the product is linear in g: its derivative along x is P x
     for have, want in ((y, P @ x.double()), (gx, P.t() @ g.double()), (gg, P @ x.double())):
         assert (have.double() - want).abs().max().item() <= 1e-5 * want.abs().max().item()
+
+
+@pytest.mark.parametrize("f", [4, 36, 64, 128])
+def test_workspace_on_an_8_byte_border(cuda, oracle, f):
+    """The C ABI asks no more of a workspace than its counter's eight bytes: hubs of few and of many pieces whose
+    partial rows start beside a 16-byte border."""
+    from jittorgeometric_b200 import _lib
+    rng = np.random.default_rng(f)
+    lens = np.concatenate([rng.integers(0, 30, 300), [16 * 8, 16 * 8 + 1, 16 * 9, 1000], rng.integers(0, 30, 300)])
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    n_in, nnz, n = 400, int(off[-1]), len(lens)
+    idx = rng.integers(0, n_in, nnz).astype(np.int32)
+    w = rng.standard_normal(nnz).astype(np.float32)
+    x = rng.standard_normal((n_in, f)).astype(np.float32)
+    off_t, idx_t, w_t, x_t = dev(off), dev(idx), dev(w), dev(x)
+    plan = cuda.ops.SpmmPlan(off_t, nnz, 16)
+    L = _lib.lib()
+    need = L.jg_aggregate_workspace_bytes(n, nnz, f, 16)
+    ws = torch.empty(need + 16, dtype=torch.uint8, device="cuda")
+    out = torch.empty((n, f), dtype=torch.float32, device="cuda")
+    assert ws.data_ptr() % 16 == 0
+    _lib.check(L.jg_aggregate_f32(out.data_ptr(), x_t.data_ptr(), idx_t.data_ptr(), off_t.data_ptr(), w_t.data_ptr(), n, n_in, f, nnz,
+                                  plan.buf.data_ptr(), 16, ws.data_ptr() + 8, need, _lib.stream_for(out)), "jg_aggregate_f32")
+    truth, scale = oracle.aggregate_f64(x, idx, off, w)
+    assert np.all(np.abs(out.cpu().numpy() - truth) <= (lens[:, None] + 4) * 2.0**-24 * scale + 1e-30)
