@@ -433,14 +433,41 @@ static HistFn hist_fn(int mode, int items) {
 // off[k] = first position whose key is >= k, for k in [0, n]; keys sorted, E entries.
 // Each thread takes four groups of four consecutive positions, a block's width apart, and issues all their loads
 // before it looks at one (285 M keys: 0.39 -> 0.38 ms; the runs of empty rows, written one by one, are the rest).
+// GAPS: rows may be empty, in long runs even (users below, items above: written by one thread, 4 M empty rows took
+// 15 ms).  Then a thread ends its run at the next multiple of kGapTile rows, and one warp per tile, in the first
+// `fill_blocks` blocks, looks up its first row's offset and writes the run that row is in up to the tile's end.
 constexpr int kOffThreads = 256;
 constexpr int kOffGroups = 4;
 constexpr int64_t kOffTile = (int64_t)kOffThreads * kOffGroups * 4;
+constexpr int kGapTile = 512;      // a power of two
+
+__device__ void fill_tile_start(const int32_t* __restrict__ key, int64_t E, int64_t n, int64_t v0, int32_t* __restrict__ off) {
+    const int lane = lane_id();
+    // first position with a key >= v0: 32 probes at once cut the range by 33
+    int64_t lo = 0, hi = E;
+    while (lo < hi) {
+        const int64_t len = hi - lo;
+        const unsigned below = __ballot_sync(kFull, __ldg(key + lo + (lane + 1) * len / 33) < v0);
+        const int c = __popc(below);        // keys are sorted: the first c probes
+        hi = c < 32 ? lo + (c + 1) * len / 33 : hi;
+        lo = c > 0 ? lo + c * len / 33 + 1 : lo;
+    }
+    int64_t last = lo < E ? (int64_t)__ldg(key + lo) : n;
+    if (last > v0 + kGapTile - 1) last = v0 + kGapTile - 1;
+    for (int64_t v = v0 + lane; v <= last; v += 32) off[v] = (int32_t)lo;
+}
+
+template <bool GAPS>
 __global__ void __launch_bounds__(kOffThreads) offsets_from_sorted_keys(const int32_t* __restrict__ key, int64_t E_host,
                                                                         const unsigned long long* __restrict__ dcount, int64_t n,
-                                                                        int32_t* __restrict__ off) {
+                                                                        int32_t* __restrict__ off, unsigned fill_blocks) {
     const int64_t E = dcount ? (int64_t)*dcount : E_host;
-    const int64_t base = (int64_t)blockIdx.x * kOffTile + 4 * threadIdx.x;
+    if (GAPS && blockIdx.x < fill_blocks) {
+        const int64_t v0 = ((int64_t)blockIdx.x * (kOffThreads / 32) + threadIdx.x / 32) * kGapTile;
+        if (v0 <= n) fill_tile_start(key, E, n, v0, off);
+        return;
+    }
+    const int64_t base = (int64_t)(GAPS ? blockIdx.x - fill_blocks : blockIdx.x) * kOffTile + 4 * threadIdx.x;
     const bool vec = reinterpret_cast<uintptr_t>(key) % 16 == 0;
     int4 k4[kOffGroups];
     int32_t before[kOffGroups];
@@ -468,12 +495,28 @@ __global__ void __launch_bounds__(kOffThreads) offsets_from_sorted_keys(const in
             const int64_t j = j0 + i;
             if (j > E) break;
             const int64_t hi = j == E ? n : k[i];
-            for (int64_t v = prev + 1; v <= hi; v++) off[v] = (int32_t)j;
+            const int64_t border = prev | (kGapTile - 1);      // the last row before the next tile
+            const int64_t end = GAPS && border < hi ? border : hi;
+            for (int64_t v = prev + 1; v <= end; v++) off[v] = (int32_t)j;
             prev = hi;
         }
     }
 }
-static inline unsigned offset_blocks(int64_t count) { return (unsigned)(count / kOffTile + 1); }   // positions 0 .. count
+// count: the entries, or their upper bound where dcount holds the number.  `gaps`: rows may be empty (with a loop on
+// every node none is).  A run of two tiles is written by one thread sooner than a search ends.
+static int launch_offsets(const int32_t* key, int64_t count, const unsigned long long* dcount, int64_t n, int32_t* off, bool gaps,
+                          cudaStream_t st) {
+    const unsigned blocks = (unsigned)(count / kOffTile + 1);              // positions 0 .. count
+    if (gaps && n >= 2 * kGapTile) {
+        const int64_t tiles = n / kGapTile + 1;                            // rows 0 .. n
+        const unsigned fill = (unsigned)((tiles + kOffThreads / 32 - 1) / (kOffThreads / 32));
+        offsets_from_sorted_keys<true><<<fill + blocks, kOffThreads, 0, st>>>(key, count, dcount, n, off, fill);
+    } else {
+        offsets_from_sorted_keys<false><<<blocks, kOffThreads, 0, st>>>(key, count, dcount, n, off, 0);
+    }
+    JG_LAUNCH_CHECK();
+    return JG_OK;
+}
 
 __global__ void set_count_kernel(unsigned long long* p, unsigned long long v) { *p = v; }
 
@@ -906,9 +949,7 @@ int jg_coo_to_compressed(const int32_t* edge_index, const float* w, int64_t n_ed
         fill_int_kernel<<<blocks_for(n_edges, 256), 256, 0, st>>>(reinterpret_cast<int*>(out_w), 0x3f800000, n_edges);
         JG_LAUNCH_CHECK();
     }
-    offsets_from_sorted_keys<<<offset_blocks(n_edges), kOffThreads, 0, st>>>(skey, n_edges, nullptr, n_nodes, out_off);
-    JG_LAUNCH_CHECK();
-    return JG_OK;
+    return launch_offsets(skey, n_edges, nullptr, n_nodes, out_off, true, st);
 }
 
 int jg_group_edges(const int32_t* node, int64_t n_edges, int64_t n_nodes, int32_t* out_edge, int32_t* out_off, float* out_ones,
@@ -939,9 +980,7 @@ int jg_group_edges(const int32_t* node, int64_t n_edges, int64_t n_nodes, int32_
         fill_int_kernel<<<blocks_for(n_edges, 256), 256, 0, st>>>(reinterpret_cast<int*>(out_ones), 0x3f800000, n_edges);
         JG_LAUNCH_CHECK();
     }
-    offsets_from_sorted_keys<<<offset_blocks(n_edges), kOffThreads, 0, st>>>(skey, n_edges, nullptr, n_nodes, out_off);
-    JG_LAUNCH_CHECK();
-    return JG_OK;
+    return launch_offsets(skey, n_edges, nullptr, n_nodes, out_off, true, st);
 }
 
 int jg_gcn_norm_compressed(const int32_t* edge_index, const float* w, int64_t n_edges, int64_t n_nodes, float fill,
@@ -1001,8 +1040,8 @@ int jg_gcn_norm_compressed(const int32_t* edge_index, const float* w, int64_t n_
     if (rc != JG_OK) return rc;
     rc = radix_sort(first, n_nodes, canonical, ws.kept, ws, csc_idx, csc_w, &skey, st, !unit, counted, ws.kept);
     if (rc != JG_OK) return rc;
-    offsets_from_sorted_keys<<<offset_blocks(cap), kOffThreads, 0, st>>>(skey, 0, ws.kept, n_nodes, csc_off);
-    JG_LAUNCH_CHECK();
+    rc = launch_offsets(skey, cap, ws.kept, n_nodes, csc_off, !add_self_loops, st);
+    if (rc != JG_OK) return rc;
     if (n_nodes > 0) {
         int* list = ws.last_loop;      // free again: the loop weights have been taken
         if (!unit) JG_CUDA(cudaMemsetAsync(ws.deg_count, 0, 2 * sizeof(int), st));
@@ -1036,8 +1075,8 @@ int jg_gcn_norm_compressed(const int32_t* edge_index, const float* w, int64_t n_
             rc = radix_sort(first, n_nodes, canonical, ws.kept, ws, csr_idx, csr_w, &skey, st, !unit, counted ? ws.matrix2 : nullptr);
         }
         if (rc != JG_OK) return rc;
-        offsets_from_sorted_keys<<<offset_blocks(cap), kOffThreads, 0, st>>>(skey, 0, ws.kept, n_nodes, csr_off);
-        JG_LAUNCH_CHECK();
+        rc = launch_offsets(skey, cap, ws.kept, n_nodes, csr_off, !add_self_loops, st);
+        if (rc != JG_OK) return rc;
         if (!weights_done) {
             rc = launch_norm_weights(skey, csr_idx, csr_w, ws.dis, ws.kept, 0, unit ? 1 : 0, cap, st);
             if (rc != JG_OK) return rc;

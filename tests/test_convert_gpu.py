@@ -210,3 +210,42 @@ def test_long_weighted_columns(cuda):
     adds = np.where(terms <= 4096, terms, terms / 2048 + 17)
     bound = (0.5 * (adds[idx] + adds[col]) + 6) * 2.0**-24
     assert np.all(np.abs(got - want) <= bound * want)
+
+
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1535, 1536, 5120, 70001])
+@pytest.mark.parametrize("where", ["none", "low", "high", "islands", "borders"])
+def test_runs_of_nodes_without_entries(cuda, n, where):
+    """Runs that are shorter than a tile of 512 nodes, cover one, many or all of them, start and end on its borders."""
+    rng = np.random.default_rng(n)
+    at = {"none": [], "low": range(min(n, 40)), "high": range(max(0, n - 40), n), "islands": range(0, n, 2500),
+          "borders": [v for b in range(0, n + 1, 2048) for v in (b - 1, b, b + 511, b + 512, b + 1023) if 0 <= v < n]}[where]
+    key = rng.permutation(np.repeat(np.array(at, np.int32), 3))
+    other = rng.integers(0, n, key.size).astype(np.int32)
+    got = cuda.cootocsr(dev(np.stack([key, other]).astype(np.int32)), None, n)
+    assert np.array_equal(host(got.row_offset), np.searchsorted(np.sort(key), np.arange(n + 1)))
+    assert np.array_equal(host(got.column_indices), other[np.argsort(key, kind="stable")])
+    csc, csr = cuda.gcn_norm_csc_csr(dev(np.stack([key, other]).astype(np.int32)), None, n, add_self_loops=False)
+    assert np.array_equal(host(csr.row_offset), np.searchsorted(np.sort(key), np.arange(n + 1)))
+    assert np.array_equal(host(csc.column_offset), np.searchsorted(np.sort(other), np.arange(n + 1)))
+
+
+def test_empty_half_of_the_ids_costs_no_more(cuda):
+    """Sources in the lower half of 8 M ids: one thread that writes the upper half's offsets takes ten times as long as
+    the whole conversion."""
+    E, n = 1_000_000, 8_000_000
+    g = torch.Generator(device="cuda").manual_seed(0)
+    src = torch.randint(0, n, (E,), device="cuda", generator=g)
+    dst = torch.randint(0, n, (E,), device="cuda", generator=g)
+    times = []
+    for s in (src, src // 2):
+        ei = torch.stack([s, dst]).to(torch.int32)
+        runs = []
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            cuda.cootocsr(ei, None, n)
+            b.record()
+            b.synchronize()
+            runs.append(a.elapsed_time(b))
+        times.append(min(runs))
+    assert times[1] <= 3 * times[0]
