@@ -772,6 +772,12 @@ __global__ void __launch_bounds__(kBlock) hub_fixup_kernel(AggArgs a) {
     }
 }
 
+// Blocks of the fix-up: one for every four hubs that a plan of `nnz` entries could list, four per SM at most.
+static unsigned fixup_blocks(int64_t nnz, int32_t chunk) {
+    const int64_t blocks = (plan_max_hubs(nnz, chunk) + 3) / 4, most = (int64_t)sm_count() * 4;
+    return (unsigned)(blocks < most ? blocks : most);
+}
+
 // Persistent grid: as many CTAs as fit on the device, but no more than the work can feed.  Every warp
 // takes at least one ticket (an atomic on one address) to learn that nothing is left, so on a small
 // graph a full grid of some ten thousand warps would spend its time queueing on that counter.
@@ -969,7 +975,7 @@ static int aggregate_impl(float* out, const float* x, const int32_t* idx, const 
     int rc = dispatch_aggregate(a, st);
     if (rc != JG_OK) return rc;
     if (plan) {
-        hub_fixup_kernel<<<sm_count() * 4, kBlock, 0, st>>>(a);
+        hub_fixup_kernel<<<fixup_blocks(nnz, chunk), kBlock, 0, st>>>(a);
         JG_LAUNCH_CHECK();
     }
     return JG_OK;
@@ -1127,7 +1133,7 @@ int jg_aggregate_f32_static(float* out, const float* x, const int32_t* idx, cons
     }
     rc = dispatch_aggregate(a, st);
     if (rc != JG_OK) return rc;
-    hub_fixup_kernel<<<sm_count() * 4, kBlock, 0, st>>>(a);
+    hub_fixup_kernel<<<fixup_blocks(nnz, chunk), kBlock, 0, st>>>(a);
     JG_LAUNCH_CHECK();
     return JG_OK;
 }
