@@ -99,6 +99,7 @@ struct AggArgs {
     unsigned long long* ticket;
     int accumulate;  // 1: add the aggregated row to what `out` already holds (old + sum)
     int64_t max_items;  // host-side upper bound on the plan's pieces (sizes the grid)
+    int64_t n_in, nnz;  // rows of x and entries (choose the kernel)
     const float* bias;  // epilogue on finished output rows: + bias[column] (null: none) ...
     const float* addend;  // [n_out, f] combined with the sum before the bias (null: none): scale * sum + add_scale * addend
     float scale, add_scale;
@@ -162,21 +163,26 @@ __device__ __forceinline__ float4 finish_value4(const AggArgs& a, float4 v, size
     return v;
 }
 
-// Row-by-row kernel of the widths above 64 (F <= 128*VPL): the warp covers one feature row, B rows are gathered per
-// batch, entries are added in stored order.
+// Row-by-row kernel (F <= 4*G*VPL).  G lanes cover one feature row, 32/G entries are gathered side by side (one "step"),
+// B steps per batch.  G = 32, all widths above 64: entries are added in stored order.  G = 8 and 16, the widths up to 64
+// where the streaming kernel below loses (see the dispatch): the lane groups' sums are added at the end.
 // EPI compiles in an epilogue (instantiations of their own: the registers of one cost the others 3 %).
-// FULL: the row is exactly 128*VPL floats wide (everything about the width folds at compile time).
+// FULL: the row is exactly 4*G*VPL floats wide (everything about the width folds at compile time).
 // !FULL: any 16-byte-aligned width up to that; lanes whose columns lie beyond it sit out.
-template <int VPL, int B, int MINB, int EPI, bool FULL>
+template <int G, int VPL, int B, int MINB, int EPI, bool FULL>
 __global__ void __launch_bounds__(kBlock, MINB) aggregate_rows_kernel(AggArgs a) {
-    const int F = FULL ? 128 * VPL : (int)a.f;
+    constexpr int EPS = 32 / G;
+    constexpr bool EXACT = G == 32;
+    const int F = FULL ? 4 * G * VPL : (int)a.f;
     __shared__ int2 s_tile[kBlock / 32][32];
     const int lane = lane_id();
+    const int sub = lane / G;
+    const int fl = lane % G;
     bool qok[VPL];
 #pragma unroll
-    for (int q = 0; q < VPL; q++) qok[q] = FULL || (lane + q * 32) * 4 < F;
+    for (int q = 0; q < VPL; q++) qok[q] = FULL || (fl + q * G) * 4 < F;
     int2* tile = s_tile[threadIdx.x / 32];
-    const char* xb = reinterpret_cast<const char*>(a.x) + lane * 16;
+    const char* xb = reinterpret_cast<const char*>(a.x) + fl * 16;
     const int64_t n_items = a.hdr ? a.hdr->n_items : 0;
     const int chunk = a.hdr ? a.hdr->chunk : 0x7fffffff;
     const int64_t total = n_items + a.n_out;
@@ -251,61 +257,76 @@ __global__ void __launch_bounds__(kBlock, MINB) aggregate_rows_kernel(AggArgs a)
                 __syncwarp();
                 const int cnt = min(32, e - j0);
                 int t = 0;
-                for (; t + B <= cnt; t += B) {  // full batches: no predicates
+                for (; t + EPS * B <= cnt; t += EPS * B) {  // full batches: no predicates
                     float4 v[B][VPL];
                     float wv[B];
 #pragma unroll
                     for (int u = 0; u < B; u++) {
-                        const int2 p = tile[t + u];
+                        const int2 p = tile[t + u * EPS + sub];
                         wv[u] = __int_as_float(p.y);
                         const float4* g = reinterpret_cast<const float4*>(xb + (size_t)(unsigned)p.x * (size_t)(F * 4));
 #pragma unroll
-                        for (int q = 0; q < VPL; q++) v[u][q] = qok[q] ? __ldg(g + q * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        for (int q = 0; q < VPL; q++) v[u][q] = qok[q] ? __ldg(g + q * G) : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
 #pragma unroll
                     for (int u = 0; u < B; u++)
 #pragma unroll
-                        for (int q = 0; q < VPL; q++) axpy4<true>(acc[q], v[u][q], wv[u]);
+                        for (int q = 0; q < VPL; q++) axpy4<EXACT>(acc[q], v[u][q], wv[u]);
                 }
                 if (t < cnt) {  // last, partial batch
+                    // Four entries per step: steps that lie wholly beyond the row are skipped by a warp-uniform test (most
+                    // rows of a power-law graph are shorter than one step; 32 columns: -6 % time).  With one or two
+                    // entries per step the test measured 5 % slower, it breaks up the batch of loads.
                     float4 v[B][VPL];
                     float wv[B];
 #pragma unroll
                     for (int u = 0; u < B; u++) {
-                        const int k = t + u;
+                        const int k = t + u * EPS + sub;
                         wv[u] = 0.f;
 #pragma unroll
                         for (int q = 0; q < VPL; q++) v[u][q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (k < cnt) {
+                        if ((EPS < 4 || t + u * EPS < cnt) && k < cnt) {
                             const int2 p = tile[k];
                             wv[u] = __int_as_float(p.y);
                             const float4* g = reinterpret_cast<const float4*>(xb + (size_t)(unsigned)p.x * (size_t)(F * 4));
 #pragma unroll
                             for (int q = 0; q < VPL; q++)
-                                if (qok[q]) v[u][q] = __ldg(g + q * 32);
+                                if (qok[q]) v[u][q] = __ldg(g + q * G);
                         }
                     }
 #pragma unroll
-                    for (int u = 0; u < B; u++)
+                    for (int u = 0; u < B; u++) {
+                        if (EPS < 4 || t + u * EPS < cnt) {
 #pragma unroll
-                        for (int q = 0; q < VPL; q++) axpy4<true>(acc[q], v[u][q], wv[u]);
+                            for (int q = 0; q < VPL; q++) axpy4<EXACT>(acc[q], v[u][q], wv[u]);
+                        }
+                    }
                 }
             }
-            {
-                float4* o = reinterpret_cast<float4*>(dst) + lane;
+#pragma unroll
+            for (int o = G; o < 32; o <<= 1)
+#pragma unroll
+                for (int q = 0; q < VPL; q++) {
+                    acc[q].x += __shfl_xor_sync(kFull, acc[q].x, o);
+                    acc[q].y += __shfl_xor_sync(kFull, acc[q].y, o);
+                    acc[q].z += __shfl_xor_sync(kFull, acc[q].z, o);
+                    acc[q].w += __shfl_xor_sync(kFull, acc[q].w, o);
+                }
+            if (sub == 0) {
+                float4* o = reinterpret_cast<float4*>(dst) + fl;
 #pragma unroll
                 for (int q = 0; q < VPL; q++) {
                     if (!qok[q]) continue;
                     if (add_old) {
-                        const float4 old = o[q * 32];
+                        const float4 old = o[q * G];
                         acc[q].x = __fadd_rn(old.x, acc[q].x);
                         acc[q].y = __fadd_rn(old.y, acc[q].y);
                         acc[q].z = __fadd_rn(old.z, acc[q].z);
                         acc[q].w = __fadd_rn(old.w, acc[q].w);
                     }
                     if (EPI != kPlain && id >= n_items)   // a finished output row (pieces of hub rows get theirs in the fix-up)
-                        acc[q] = finish_value4<EPI>(a, acc[q], (size_t)(id - n_items) * F + 4 * (lane + q * 32), 4 * (lane + q * 32));
-                    __stcs(o + q * 32, acc[q]);
+                        acc[q] = finish_value4<EPI>(a, acc[q], (size_t)(id - n_items) * F + 4 * (fl + q * G), 4 * (fl + q * G));
+                    __stcs(o + q * G, acc[q]);
                 }
             }
         }
@@ -815,19 +836,19 @@ static int launch_persistent(K kern, int* blocks_per_sm, const AggArgs& a, cudaS
 
 static int epilogue_of(const AggArgs& a) { return a.addend ? kCombine : (a.bias || a.relu) ? kBiasAct : kPlain; }
 
-template <int VPL, int B, int MINB, bool FULL>
+template <int G, int VPL, int B, int MINB, bool FULL>
 static int launch_rows_as(const AggArgs& a, cudaStream_t st) {
     static int bps[3] = {0, 0, 0};
     switch (epilogue_of(a)) {
-        case kPlain: return launch_persistent(aggregate_rows_kernel<VPL, B, MINB, kPlain, FULL>, &bps[0], a, st);
-        case kBiasAct: return launch_persistent(aggregate_rows_kernel<VPL, B, MINB, kBiasAct, FULL>, &bps[1], a, st);
-        default: return launch_persistent(aggregate_rows_kernel<VPL, B, MINB, kCombine, FULL>, &bps[2], a, st);
+        case kPlain: return launch_persistent(aggregate_rows_kernel<G, VPL, B, MINB, kPlain, FULL>, &bps[0], a, st);
+        case kBiasAct: return launch_persistent(aggregate_rows_kernel<G, VPL, B, MINB, kBiasAct, FULL>, &bps[1], a, st);
+        default: return launch_persistent(aggregate_rows_kernel<G, VPL, B, MINB, kCombine, FULL>, &bps[2], a, st);
     }
 }
-// a narrower 16-byte-aligned width than 128 * VPL runs on the same lane layout
-template <int VPL, int B, int MINB>
+// a narrower 16-byte-aligned width than 4 * G * VPL runs on the same lane layout
+template <int G, int VPL, int B, int MINB>
 static int launch_rows(const AggArgs& a, cudaStream_t st) {
-    return a.f == 128 * VPL ? launch_rows_as<VPL, B, MINB, true>(a, st) : launch_rows_as<VPL, B, MINB, false>(a, st);
+    return a.f == 4 * G * VPL ? launch_rows_as<G, VPL, B, MINB, true>(a, st) : launch_rows_as<G, VPL, B, MINB, false>(a, st);
 }
 
 template <int F>
@@ -854,15 +875,22 @@ static int dispatch_aggregate(const AggArgs& a, cudaStream_t st) {
     const bool vec_ok = (f % 4 == 0) && ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.out) |
                                           reinterpret_cast<uintptr_t>(a.partial) |
                                           reinterpret_cast<uintptr_t>(a.addend)) % 16 == 0);
-    // widths up to 64 normally put two to four entries of a row side by side in one warp and add the
-    // lane groups' partial sums at the end; an ordered sum takes the narrow kernel (F <= 32) or the
-    // 128-column layout with idle lanes (F <= 64) instead
-    // (with the lane groups' partial sums added at the end the streaming kernel differs from the sequential
-    // sum by rounding anyway: it uses one fused multiply-add per term)
-    // The streaming kernel against the row-by-row one on 8 or 16 lanes, us: 32 columns, 62 M entries 855 -> 780; 64
-    // columns, 132 M 3900 -> 3150; 48 columns, 2.5 M 141 -> 99; 40 columns, 4.9 M 160 -> 152.  Above 64 columns, where a
-    // step is one entry and the sum is in stored order, it was slower (72 columns, 18 M entries: 780 -> 980): unused there.
-    if (vec_ok && !a.ordered) {
+    // Widths of 32 and 36 to 64 put two or four entries of a row side by side in one warp and add the lane groups'
+    // partial sums at the end: that differs from the sequential sum by rounding anyway, so it uses one fused
+    // multiply-add per term.  An ordered sum takes the narrow kernel (F <= 32) or the 128-column layout with idle lanes.
+    // Row by row or streaming, us (R-MAT unless said):
+    //   below eight rows a warp the streaming kernel's start is not paid back: 2.7 k rows, 48 columns, 27 k entries 12.4
+    //   against 16.5, 20 k rows, 100 k entries 26 against 30; at 60 k rows it is 56 against 41;
+    //   rows of 40 and more entries keep the row kernel's batches full, and out of L2 the streaming kernel is bound by
+    //   instructions (40 columns, 170 k rows, 71 entries a row 235 against 278, 38 entries 200 against 175; evenly spread
+    //   sources, 300 k rows, 40 entries 220 against 257); with all lanes at work, at 64 columns, the line is at 48 (170 k
+    //   rows, 71 entries 257 against 274, 38 entries 211 against 174);
+    //   where x does not fit L2 the streaming kernel hides more latency: 64 columns, 2 M rows, 132 M entries 3900
+    //   against 3150; at 32 columns it wins for long rows as well (1 M rows, 62 M entries 855 against 780).
+    if (vec_ok && !a.ordered && f >= 32 && f <= 64) {
+        const bool few = a.n_out < (int64_t)sm_count() * 256;
+        const bool lengthy = f > 32 && a.nnz >= a.n_out * (f < 64 ? 40 : 48) && a.n_in * f * 4 <= ((int64_t)(f < 64 ? 100 : 64) << 20);
+        if (few || lengthy) return f == 32 ? launch_rows_as<8, 1, 8, 4, true>(a, st) : launch_rows<16, 1, 8, 4>(a, st);
         switch (f) {
             case 32: return launch_stream<32>(a, st);
             case 36: return launch_stream<36>(a, st);
@@ -875,10 +903,9 @@ static int dispatch_aggregate(const AggArgs& a, cudaStream_t st) {
             case 64: return launch_stream<64>(a, st);
         }
     }
-    if (vec_ok && f > 32 && f <= 64) return launch_rows<1, 8, 4>(a, st);
-    if (vec_ok && f > 64 && f <= 128) return launch_rows<1, 8, 4>(a, st);
-    if (vec_ok && f > 128 && f <= 256) return launch_rows<2, 4, 4>(a, st);
-    if (vec_ok && f > 256 && f <= 512) return launch_rows<4, 2, 3>(a, st);
+    if (vec_ok && f > 32 && f <= 128) return launch_rows<32, 1, 8, 4>(a, st);
+    if (vec_ok && f > 128 && f <= 256) return launch_rows<32, 2, 4, 4>(a, st);
+    if (vec_ok && f > 256 && f <= 512) return launch_rows<32, 4, 2, 3>(a, st);
     if (f <= 32) {   // narrow rows (any alignment): several rows per warp
         if (f <= 4) return launch_narrow<4>(a, st);
         if (f <= 8) return launch_narrow<8>(a, st);
@@ -953,6 +980,7 @@ static int aggregate_impl(float* out, const float* x, const int32_t* idx, const 
 
     AggArgs a = {};
     a.out = out; a.x = x; a.idx = idx; a.off = off; a.w = w; a.n_out = n_out; a.f = f;
+    a.n_in = n_in; a.nnz = nnz;
     a.accumulate = accumulate;
     a.bias = bias;
     a.relu = relu;
@@ -1112,6 +1140,7 @@ int jg_aggregate_f32_static(float* out, const float* x, const int32_t* idx, cons
     Carver c(base);
     AggArgs a = {};
     a.out = out; a.x = x; a.idx = idx; a.off = off; a.w = w; a.n_out = n_out; a.f = f;
+    a.n_in = n_in; a.nnz = nnz;
     a.ticket = c.take<unsigned long long>(1);
     PlanView v = plan_view(c.take<unsigned char>(plan_bytes), nnz, chunk, nullptr);
     a.hdr = v.hdr; a.hub_row = v.hub_row; a.hub_first = v.hub_first; a.item_hub = v.item_hub; a.item_k = v.item_k;

@@ -329,3 +329,56 @@ def test_workspace_on_an_8_byte_border(cuda, oracle, f):
                                   plan.buf.data_ptr(), 16, ws.data_ptr() + 8, need, _lib.stream_for(out)), "jg_aggregate_f32")
     truth, scale = oracle.aggregate_f64(x, idx, off, w)
     assert np.all(np.abs(out.cpu().numpy() - truth) <= (lens[:, None] + 4) * 2.0**-24 * scale + 1e-30)
+
+
+@pytest.mark.parametrize("mode", ["plain", "epilogue", "accumulate", "combine"])
+@pytest.mark.parametrize("n,f", [(n, f) for n in (60001, 130003) for f in (32, 36, 40, 44, 48, 52, 56, 60, 64)] +
+                         [(930001, f) for f in (32, 40, 64)])
+def test_several_rows_a_ticket(cuda, n, f, mode):
+    """2, 4 and 8 rows a ticket (the last ticket cut short): rows of 0 to 34 entries in every order, runs of empty rows, hub
+    rows between rows of the same ticket.  The same rows in calls too small for that are walked row by row, the sums in
+    the same order: equal bit for bit.  Those are checked against float64 above."""
+    rng = np.random.default_rng(n + f)
+    lens = rng.integers(0, 7, n)
+    for at in range(0, n - 200, n // 9):
+        lens[at:at + 35], lens[at + 35:at + 75], lens[at + 75:at + 82] = np.arange(35), 0, [63, 64, 65, 200, 0, 129, 7]
+    lens[rng.integers(0, n, 200)] = 300
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    n_in, nnz = 5000, int(off[-1])
+    gen = torch.Generator(device="cuda").manual_seed(f)
+    idx = torch.randint(1, n_in, (nnz,), device="cuda", generator=gen, dtype=torch.int32)
+    w = torch.randn(nnz, device="cuda", generator=gen)
+    x = torch.randn((n_in, f), device="cuda", generator=gen)
+    x[0] = float("inf")          # no entry names it
+    other, bias = torch.randn((n, f), device="cuda", generator=gen), torch.randn(f, device="cuda", generator=gen)
+
+    def call(a, b):
+        o = dev(off[a:b + 1])
+        kw = {"plain": {}, "epilogue": dict(bias=bias, relu=True), "accumulate": dict(out=other[a:b].clone(), accumulate=True),
+              "combine": dict(addend=other[a:b], scale=0.9, add_scale=0.1)}[mode]
+        return cuda.ops.segment_aggregate(x, idx, o, w, plan=cuda.ops.SpmmPlan(o, nnz, 64), **kw)
+
+    got = call(0, n)
+    for a in range(0, n, 30000):
+        b = min(a + 30000, n)
+        assert torch.equal(got[a:b], call(a, b))
+    assert torch.isfinite(got).all()
+
+
+@pytest.mark.parametrize("f", [36, 48, 60, 64])
+def test_long_rows_on_either_kernel(cuda, f):
+    """Rows of some 40 to 80 entries are walked row by row while x fits L2 and streamed beyond that: the same rows of a
+    short and of a long x take the two kernels.  Equal bit for bit."""
+    n, n_in = 40009, 3000
+    rng = np.random.default_rng(f)
+    lens = rng.integers(40, 56, n) if f < 64 else rng.integers(56, 80, n)
+    lens[rng.integers(0, n, 50)] = 700
+    off = dev(np.concatenate([[0], np.cumsum(lens)]).astype(np.int32))
+    nnz = int(off[-1])
+    gen = torch.Generator(device="cuda").manual_seed(f)
+    idx = torch.randint(0, n_in, (nnz,), device="cuda", generator=gen, dtype=torch.int32)
+    w, x = torch.randn(nnz, device="cuda", generator=gen), torch.randn((n_in, f), device="cuda", generator=gen)
+    far = torch.zeros((1_000_000, f), device="cuda")
+    far[:n_in] = x
+    plan = cuda.ops.SpmmPlan(off, nnz, 256)
+    assert torch.equal(cuda.ops.segment_aggregate(x, idx, off, w, plan=plan), cuda.ops.segment_aggregate(far, idx, off, w, plan=plan))
