@@ -744,12 +744,21 @@ static int gemm_impl(float* out, void* out_half, const float* x, const float* wt
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int32_t* error = static_cast<int32_t*>(workspace);
     if (clear_error) JG_CUDA(cudaMemsetAsync(error, 0, sizeof(int32_t), st));
-    // Column tiles of 256 (128 when the fp16 copy needs its own staging slabs in shared memory), x read once per
-    // tile; halved, down to 64, while the tiles do not reach every SM: a citation graph's 2708 x 1433 -> 256 is
-    // 22 row tiles, and the time of one is set by how many rows of both operands it has to fetch per step.
+    // Column tiles of 256 (128 when the fp16 copy needs its own staging slabs in shared memory), x read once per tile.
+    // While all tiles are one wave of CTAs (one per SM) the time is that of one tile, and that is set by the rows of both
+    // operands it fetches per step: then tiles of 128 or 64, as long as those are one wave too.  2708 x 1433 -> 256, 22 row
+    // tiles: 123 us with one column tile, 55 with four.  A second wave costs more than the narrower tile saves:
+    // 75 row tiles, 256 -> 256 9.4 us with one column tile, 13 with two; 1433 -> 130 95 against 120.
     int64_t tile_w = out_half ? 128 : 256;
     const int64_t row_tiles = (n_rows + kTileM - 1) / kTileM;
-    while (tile_w > 64 && m > tile_w / 2 && row_tiles * ((m + tile_w - 1) / tile_w) < sm_count()) tile_w /= 2;
+    for (int64_t w = tile_w / 2; w >= 64; w /= 2)
+        if (w < m && row_tiles * ((m + w - 1) / w) <= sm_count()) tile_w = w;
+    // Rows without a 16-byte pitch are stored by plain stores, and with a short k those are most of a tile's time: tiles of
+    // 64 in two waves then (64 -> 130, 60 row tiles: 15 us in tiles of 128, 9.7).
+    if (m % 4 && m > 128 && k <= 256 && tile_w == 128) tile_w = 64;
+    // tiles of equal width, whole 32-column stores (602 -> 300 in tiles of 256 and 44 fetched 256 rows for both)
+    const int64_t col_tiles = (m + tile_w - 1) / tile_w;
+    tile_w = ((m + col_tiles - 1) / col_tiles + 31) / 32 * 32;
     if (tile_w > m) tile_w = m;
     return gemm_launch(out, x, wt, bias, n_rows, k, tile_w, m, relu, error, st, static_cast<__half*>(out_half));
 }

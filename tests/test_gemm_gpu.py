@@ -243,22 +243,45 @@ def test_fp32_row_reduction_tile_edges(cuda, M, N, K):
     assert torch.equal(got, cuda.ops.matmul_f32(a, b, trans_a=True))
 
 
-@pytest.mark.parametrize("m", [47, 65, 100, 130, 256, 300])
+@pytest.mark.parametrize("m", [47, 65, 100, 128, 130, 256, 300, 512])
 @pytest.mark.parametrize("k", [33, 64, 602])
 def test_column_tiles_of_short_inputs(cuda, k, m):
-    """With few rows the output is cut into column tiles of 64 or 128; every value is the same sum as in the one-tile
-    product of the same rows among many."""
+    """Few rows are cut into column tiles of 64 and more columns (1, 200, 5000 rows: 64; 9000: 128 for 256 and 64 for up
+    to 130 with a short k; 300 and 512 in equal tiles), many rows are not up to 256; every value is the same sum either way."""
     g = torch.Generator(device="cuda").manual_seed(k + m)
     x = torch.randn((40000, k), device="cuda", generator=g)
     w = torch.randn((k, m), device="cuda", generator=g)
     bias = torch.randn(m, device="cuda", generator=g)
     many = cuda.ops.linear_tf32(x, w, bias=bias, relu=True)
-    for n in (1, 200, 5000):
+    for n in (1, 200, 5000, 9000, 18800):
         few = cuda.ops.linear_tf32(x[:n].contiguous(), w, bias=bias, relu=True, check_status=True)
         assert torch.equal(few, many[:n])
     want = torch.relu(x.double() @ w.double() + bias.double())
     scale = x.abs().double() @ w.abs().double() + bias.abs().double()
     assert ((many.double() - want).abs() / scale).max().item() <= 2e-3
+
+
+@pytest.mark.parametrize("n,k,m", [(18800, 256, 256), (12800, 64, 200)])
+def test_column_tiles_make_no_second_wave(cuda, n, k, m):
+    """147 and 100 row tiles are one wave of one column tile, 149 are two: fewer rows take less time."""
+    x, w = torch.randn((149 * 128, k), device="cuda"), torch.randn((k, m), device="cuda")
+    wt = w.t().contiguous()
+
+    def time(rows):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        best = 1e9
+        for _ in range(5):
+            torch.cuda._sleep(400000)      # the launches queue up behind it
+            a.record()
+            for _ in range(10):
+                cuda.ops.linear_tf32(x[:rows], w, weight_t=wt)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    time(n)
+    assert time(n) <= time(149 * 128)
 
 
 @pytest.mark.parametrize("n", [1, 31, 33, 5000])
