@@ -107,8 +107,9 @@ __global__ void __launch_bounds__(kEdgeBlock) edge_to_vertex_dst_kernel(float* _
 // V values (4, 2 or 1: what C and both bases are aligned to) per atomic instruction.  The message is
 // read once, so the bound would be DRAM; in fact it is L2's fp32 adders (7 M edges of 64 columns: 1.27 ms with
 // one value per instruction, 1.08 ms with four, 0.28 ms for the bytes).
-// G lanes share an edge's row (a power of two, at least the row's vectors where 32 lanes suffice); a group
-// walks kEdgesPerGroup consecutive edges, whose loads are all issued before the first reduction.
+// `lanes_per_row` lanes, at most 32, share an edge's row, as many as leave none idle (5 columns: 5 lanes 9.5 us for 0.5 M
+// edges, 8 lanes 11.9; 33 columns: 17 lanes twice, 32 lanes 63 us); a group walks kEdgesPerGroup consecutive edges, whose
+// loads are all issued before the first reduction.
 template <int V> struct AtomVec;
 template <> struct AtomVec<1> { typedef float T; };
 template <> struct AtomVec<2> { typedef float2 T; };
@@ -119,9 +120,10 @@ __global__ void __launch_bounds__(kEdgeBlock) edge_to_vertex_src_kernel(float* _
                                                                         const int32_t* __restrict__ idx, int64_t E, int64_t C,
                                                                         int lanes_per_row) {
     typedef typename AtomVec<V>::T T;
-    const int64_t group = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / lanes_per_row;
-    const int64_t n_groups = (int64_t)gridDim.x * blockDim.x / lanes_per_row;
+    const int64_t group = (int64_t)blockIdx.x * (kEdgeBlock / lanes_per_row) + threadIdx.x / lanes_per_row;
+    const int64_t n_groups = (int64_t)gridDim.x * (kEdgeBlock / lanes_per_row);
     const int gl = threadIdx.x % lanes_per_row;
+    if (threadIdx.x >= kEdgeBlock / lanes_per_row * lanes_per_row) return;
     const int64_t vecs = C / V;
     for (int64_t e0 = group * kEdgesPerGroup; e0 < E; e0 += n_groups * kEdgesPerGroup) {
         int32_t dst[kEdgesPerGroup];
@@ -702,10 +704,10 @@ int jg_edge_to_vertex_f32(float* out, const float* msg, const int32_t* idx, cons
         if (n_edges > 0) {
             const uintptr_t both = reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(msg);
             const int v = (c % 4 == 0 && both % 16 == 0) ? 4 : (c % 2 == 0 && both % 8 == 0) ? 2 : 1;
-            int g = 1;
-            while (g < 32 && g < c / v) g *= 2;
-            const int64_t groups = (n_edges + kEdgesPerGroup - 1) / kEdgesPerGroup;
-            const unsigned grid = grid_for_warps((groups * g + 31) / 32);
+            const int64_t sweeps = (c / v + 31) / 32;
+            const int g = (int)((c / v + sweeps - 1) / sweeps);
+            const int64_t groups = (n_edges + kEdgesPerGroup - 1) / kEdgesPerGroup, per_block = kEdgeBlock / g;
+            const unsigned grid = grid_for_warps((groups + per_block - 1) / per_block * (kEdgeBlock / 32));
             if (v == 4) edge_to_vertex_src_kernel<4><<<grid, kEdgeBlock, 0, st>>>(out, msg, idx, n_edges, c, g);
             else if (v == 2) edge_to_vertex_src_kernel<2><<<grid, kEdgeBlock, 0, st>>>(out, msg, idx, n_edges, c, g);
             else edge_to_vertex_src_kernel<1><<<grid, kEdgeBlock, 0, st>>>(out, msg, idx, n_edges, c, g);

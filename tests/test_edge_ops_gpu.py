@@ -224,9 +224,9 @@ def test_gat_layer_fused_and_unfused_agree(cuda):
 
 
 @pytest.mark.parametrize("edges", [1, 3, 5, 4099])
-@pytest.mark.parametrize("c", [1, 2, 3, 4, 6, 30, 64, 126, 132, 260])
+@pytest.mark.parametrize("c", [1, 2, 3, 4, 5, 6, 17, 30, 33, 64, 65, 126, 132, 260])
 def test_scatter_to_edge_backward_by_source(cuda, c, edges):
-    """Vector reductions of 4, 2 and 1 values, edge counts that end inside a group of edges.  A sum of k terms in
+    """Vector reductions of 4, 2 and 1 values, rows of one lane to several sweeps of them, edge counts that end inside a group.  A sum of k terms in
     any order is off by at most (k - 1) * 2^-24 of the sum of magnitudes."""
     n, rng = 37, np.random.default_rng(c + edges)
     idx, off = random_csc(rng, n, edges)
