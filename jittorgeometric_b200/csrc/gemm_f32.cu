@@ -260,8 +260,23 @@ static void launch_tn(const SgemmArgs& g, cudaStream_t st) {
     else launch_tn_b<TN, 1>(g, bv, grid, smem, st);
 }
 
-// C = sum of the slices' partial tiles in slice order (+ bias, ReLU).
-// 32 outputs per block; eight groups of threads add an eighth of the slices each, in order, and the eighths are
+// C = sum of the slices' partial tiles in slice order (+ bias, ReLU), one thread per output.
+__global__ void __launch_bounds__(256) sgemm_reduce_few_kernel(float* __restrict__ c, const float* __restrict__ partial, int64_t M,
+                                                               int64_t N, int64_t ldc, int slices, const float* __restrict__ bias,
+                                                               int relu) {
+    const size_t mn = (size_t)(M * N);
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < M * N; t += (int64_t)gridDim.x * blockDim.x) {
+        float v = __ldg(partial + t);
+#pragma unroll 8
+        for (int s = 1; s < slices; s++) v = __fadd_rn(v, __ldg(partial + (size_t)s * mn + t));
+        const int64_t i = t / N, j = t - i * N;
+        if (bias) v += __ldg(bias + j);
+        if (relu) v = fmaxf(v, 0.f);
+        c[i * ldc + j] = v;
+    }
+}
+
+// The same for many slices of few outputs.  32 outputs per block; eight groups of threads add an eighth of the slices each, in order, and the eighths are
 // added in order: with one thread per output, 148 slices of a 128 x 128 gradient were a chain of 148 loads.
 __global__ void __launch_bounds__(256) sgemm_reduce_kernel(float* __restrict__ c, const float* __restrict__ partial, int64_t M,
                                                            int64_t N, int64_t ldc, int slices, const float* __restrict__ bias, int relu) {
@@ -292,17 +307,24 @@ __global__ void __launch_bounds__(256) sgemm_reduce_kernel(float* __restrict__ c
     }
 }
 
-static unsigned reduce_blocks(int64_t M, int64_t N) {
-    int64_t blocks = (M * N + 31) / 32;
+// The second kernel's barriers cost more than the chain they cut where the first fills the device by itself: from 2^17
+// outputs on, or from 2^15 with two loads or less in each of the groups (2708 x 256 outputs, two slices: 5 us against 15;
+// 1432 x 256, three: 4 against 11; 64 x 64, eight: 3 against 2).
+static int launch_reduce(float* c, const float* partial, int64_t M, int64_t N, int64_t ldc, int slices, const float* bias, int relu,
+                         cudaStream_t st) {
+    const bool few = M * N >= (int64_t)1 << 17 || (M * N > (int64_t)1 << 15 && slices <= 16);
+    const int64_t per_block = few ? 256 : 32;
+    int64_t blocks = (M * N + per_block - 1) / per_block;
     if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
-    return (unsigned)(blocks < 1 ? 1 : blocks);
+    if (few) sgemm_reduce_few_kernel<<<(unsigned)blocks, 256, 0, st>>>(c, partial, M, N, ldc, slices, bias, relu);
+    else sgemm_reduce_kernel<<<(unsigned)blocks, 256, 0, st>>>(c, partial, M, N, ldc, slices, bias, relu);
+    JG_LAUNCH_CHECK();
+    return JG_OK;
 }
 
 // Used by the tensor-core weight gradient as well: c[M, N] = sum of `slices` partial results, in order.
 int reduce_slices(float* c, const float* partial, int64_t M, int64_t N, int slices, cudaStream_t st) {
-    sgemm_reduce_kernel<<<reduce_blocks(M, N), 256, 0, st>>>(c, partial, M, N, N, slices, nullptr, 0);
-    JG_LAUNCH_CHECK();
-    return JG_OK;
+    return launch_reduce(c, partial, M, N, N, slices, nullptr, 0, st);
 }
 
 static int sgemm_slices(int64_t M, int64_t N, int64_t K) {
@@ -365,11 +387,7 @@ int jg_gemm_f32(float* c, const float* a, const float* b, const float* bias, int
         sgemm_kernel<<<grid, 256, 0, st>>>(g);
     }
     JG_LAUNCH_CHECK();
-    if (g.slices > 1) {
-        sgemm_reduce_kernel<<<reduce_blocks(M, N), 256, 0, st>>>(c, static_cast<const float*>(workspace), M, N, ldc, g.slices, bias, relu);
-        JG_LAUNCH_CHECK();
-    }
-    return JG_OK;
+    return g.slices > 1 ? launch_reduce(c, static_cast<const float*>(workspace), M, N, ldc, g.slices, bias, relu, st) : JG_OK;
 }
 
 }  // extern "C"
