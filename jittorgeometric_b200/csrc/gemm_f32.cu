@@ -196,21 +196,36 @@ __global__ void __launch_bounds__(256, 2) sgemm_tn_kernel(SgemmArgs g) {
     const bool single = g.slices == 1;
     float* out = single ? g.c : g.c + (size_t)blockIdx.z * (size_t)g.M * (size_t)g.N;
     const int64_t ld = single ? g.ldc : g.N;
+    const bool vec = g.N % 4 == 0 && ld % 4 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0;
+    auto finish = [&](int r, int c, int64_t j) {
+        const unsigned long long p = acc[r / 2][c];
+        float v = __uint_as_float((unsigned)(r % 2 ? p >> 32 : p));
+        if (single) {
+            if (g.bias) v += __ldg(g.bias + j);
+            if (g.relu) v = fmaxf(v, 0.f);
+        }
+        return v;
+    };
 #pragma unroll
     for (int r = 0; r < 8; r++) {
         const int64_t i = i0 + ty * 8 + r;
         if (i >= g.M) continue;
+        if constexpr (TN % 4 == 0) {
+            if (vec) {       // four columns of a thread lie side by side
+#pragma unroll
+                for (int c = 0; c < TN; c += 4) {
+                    const int64_t j = j0 + (c / 4) * 64 + tx * 4;
+                    if (j < g.N) *reinterpret_cast<float4*>(out + i * ld + j) =
+                        make_float4(finish(r, c, j), finish(r, c + 1, j + 1), finish(r, c + 2, j + 2), finish(r, c + 3, j + 3));
+                }
+                continue;
+            }
+        }
 #pragma unroll
         for (int c = 0; c < TN; c++) {
             const int64_t j = j0 + (TN % 4 == 0 ? (c / 4) * 64 + tx * 4 + c % 4 : c * 16 + tx);
             if (j >= g.N) continue;
-            const unsigned long long p = acc[r / 2][c];
-            float v = __uint_as_float((unsigned)(r % 2 ? p >> 32 : p));
-            if (single) {
-                if (g.bias) v += __ldg(g.bias + j);
-                if (g.relu) v = fmaxf(v, 0.f);
-            }
-            out[i * ld + j] = v;
+            out[i * ld + j] = finish(r, c, j);
         }
     }
 }
@@ -236,6 +251,15 @@ static int tn_row_slices(int64_t M, int64_t N, int64_t K) {
     const int64_t most = (K + 4 * kTnK - 1) / (4 * kTnK);                // at least four steps each
     if (want > most) want = most;
     return want < 1 ? 1 : (int)want;
+}
+
+// A few CTAs of 128 x 128 outputs each take longer than the many 64 x 64 tiles of the kernel above: 16 rows, 1433 x 256
+// columns 6.2 us against 4.0, 1000 rows, 47 x 256 12.6 against 11.0.  From a quarter of the SMs on, and with narrower
+// tiles at any count, it is the faster one (128 rows, 1433 x 256, 48 CTAs: 14.6 both; 500 rows, 64 x 64, 8 CTAs: 8.8 against 10.9).
+static bool tn_pays(int64_t M, int64_t N, int64_t K) {
+    const int cols = tn_cols(N);
+    const int64_t tiles = ((M + kTnM - 1) / kTnM) * ((N + 16 * cols - 1) / (16 * cols));
+    return cols < 8 || tiles * tn_row_slices(M, N, K) * 4 >= sm_count();
 }
 
 static int copy_floats(const float* p, int64_t pitch) {
@@ -360,7 +384,7 @@ int jg_gemm_f32(float* c, const float* a, const float* b, const float* bias, int
     SgemmArgs g = {};
     g.a = a; g.b = b; g.bias = bias; g.M = M; g.N = N; g.K = K;
     g.sa0 = sa0; g.sa1 = sa1; g.sb0 = sb0; g.sb1 = sb1; g.ldc = ldc; g.relu = relu;
-    const bool tn = sa0 == 1 && sb1 == 1 && K > 0 && sa1 >= M && sb0 >= N;   // both operands along their rows
+    const bool tn = sa0 == 1 && sb1 == 1 && K > 0 && sa1 >= M && sb0 >= N && tn_pays(M, N, K);   // both operands along their rows
     static_assert(kTnK == kBK, "one rounding of the slices serves both kernels");
     g.slices = K > 0 ? (tn ? tn_row_slices(M, N, K) : sgemm_slices(M, N, K)) : 1;
     g.k_slice = ((K + g.slices - 1) / g.slices + kBK - 1) / kBK * kBK;
