@@ -299,3 +299,41 @@ def test_masked_gradient_and_column_sums(cuda, n, f):
     grad[0, 0], y[0, 0] = float("inf"), -1.0
     gm, gsum = cuda.ops._epilogue_grad(grad, y, True)
     assert torch.isnan(gm[0, 0]) and torch.isnan(gsum[0])
+
+
+@pytest.mark.parametrize("n", [1, 33, 8191, 8192, 20001])
+@pytest.mark.parametrize("f", [1, 7, 47, 130, 514, 602, 1028])
+def test_masked_gradient_splits(cuda, n, f):
+    """Both thread counts, slabs of columns, rows of 1, 2 and 4 values a lane, and bases beside a 16-byte border: the mask
+    is exact with and without the sums, a column's sum passes at most n additions in any order."""
+    g = torch.Generator(device="cuda").manual_seed(n + f)
+    shifted = lambda: torch.randn(n * f + 1, device="cuda", generator=g)[1:].view(n, f)
+    for grad, y in ((torch.randn((n, f), device="cuda", generator=g), torch.randn((n, f), device="cuda", generator=g)),
+                    (shifted(), shifted())):
+        want = grad * (y > 0)
+        gm, gsum = cuda.ops._epilogue_grad(grad, y, True)
+        alone, none = cuda.ops._epilogue_grad(grad, y, False)
+        assert none is None and torch.equal(gm, want) and torch.equal(alone, want)
+        total = cuda.ops._epilogue_grad(grad, None, True)[1]
+        for have, of in ((gsum, want), (total, grad)):
+            assert ((have.double() - of.double().sum(0)).abs() <= n * 2.0**-24 * of.double().abs().sum(0)).all()
+
+
+@pytest.mark.parametrize("n,f", [(64, 4096), (170000, 130)])
+def test_mask_of_few_wide_and_unaligned_rows_is_no_slower_than_two_passes(cuda, n, f):
+    grad, y = torch.randn((n, f), device="cuda"), torch.randn((n, f), device="cuda")
+
+    def time(fn):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        best = 1e9
+        for _ in range(6):
+            torch.cuda._sleep(800000)      # the launches queue up behind it
+            a.record()
+            for _ in range(10):
+                fn()
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    assert time(lambda: cuda.ops._epilogue_grad(grad, y, False)) <= time(lambda: grad * (y > 0))
