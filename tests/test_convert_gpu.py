@@ -249,3 +249,20 @@ def test_empty_half_of_the_ids_costs_no_more(cuda):
             runs.append(a.elapsed_time(b))
         times.append(min(runs))
     assert times[1] <= 3 * times[0]
+
+
+@pytest.mark.parametrize("E", [31, 2049, 128 * 2048 + 1, (1 << 21) + 4095])
+@pytest.mark.parametrize("order", ["sorted", "one", "runs", "mixed"])
+def test_lists_with_runs_of_equal_keys(cuda, oracle, E, order):
+    """Warps whose first 32 digits are few runs are ranked by match masks, the others by votes: all of them the one, all the
+    other, and both in one tile, with 8 and with 16 entries a thread; a row of the output is its entries in list order."""
+    rng = np.random.default_rng(E)
+    n = 70001
+    dst = {"sorted": lambda: np.sort(rng.integers(0, n, E)), "one": lambda: np.full(E, 4711),
+           "runs": lambda: np.repeat(rng.integers(0, n, E // 5 + 1), 5)[:E],
+           "mixed": lambda: np.where(np.arange(E) // 256 % 2, np.arange(E) // 3 % n, rng.integers(0, n, E))}[order]()
+    ei = np.stack([rng.integers(0, n, E), dst]).astype(np.int32)
+    for got, fn in ((cuda.cootocsr(dev(ei), None, n), oracle.coo_to_csr), (cuda.cootocsc(dev(ei), None, n), oracle.coo_to_csc)):
+        idx, off, _ = fn(ei, np.ones(E, np.float32), n)
+        g_idx, g_off = (got.column_indices, got.row_offset) if fn is oracle.coo_to_csr else (got.row_indices, got.column_offset)
+        assert np.array_equal(host(g_off), off) and np.array_equal(host(g_idx), idx)
