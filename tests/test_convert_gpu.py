@@ -197,10 +197,11 @@ def test_long_weighted_columns(cuda):
     sizes = [4095, 4096, 40961, 63, 64, 95]     # with the loop: a warp's last, a block's first, a thread's last, a warp's first
     dst = np.concatenate([np.full(k, h) for h, k in zip(hubs, sizes)] + [rng.integers(100, 300, 2000)])
     src = rng.integers(0, n, dst.size)
-    dst, src = np.where(src == dst, (dst + 1) % n, dst), src
+    src = np.where(src == dst, (dst + 1) % n, src)
     w = (rng.random(dst.size) + 0.5).astype(np.float32)
     csc, _ = cuda.gcn_norm_csc_csr(dev(np.stack([src, dst]).astype(np.int32)), dev(w), n)
     off, idx, got = host(csc.column_offset), host(csc.row_indices), host(csc.edge_weight).astype(np.float64)
+    assert np.array_equal(np.diff(off)[hubs], np.array(sizes) + 1)
     order = np.argsort(np.concatenate([dst, np.arange(n)]), kind="stable")
     raw = np.concatenate([w, np.ones(n, np.float32)]).astype(np.float64)[order]
     col = np.repeat(np.arange(n), np.diff(off))
