@@ -21,7 +21,7 @@ DEFAULT_CHUNK = int(os.environ.get("JG_SPMM_CHUNK", "1024"))
 SMALL_GRAPH_NNZ = 1 << 20
 SMALL_GRAPH_CHUNK = int(os.environ.get("JG_SPMM_SMALL_CHUNK", "64"))
 FEW_ROWS = 1 << 19
-GROUP_VALUES, GROUP_COLUMNS = 1 << 26, 24
+GROUP_VALUES = 1 << 26
 FEW_ROWS_CHUNK = int(os.environ.get("JG_SPMM_FEW_ROWS_CHUNK", "256"))
 
 
@@ -499,12 +499,19 @@ def _scatter_to_edge(x, csc, flag):
     return out
 
 
-def _group_by_source(n_edges, c):
+def _group_by_source(n_edges, n_nodes, c):
     """Whether the sum per source groups the edges first (:func:`_sum_by_source`) or reduces into L2 in edge order.
-    The reductions cost per value, the grouping per edge: 7 M edges 64 columns 1.13 against 0.60 ms, 32 columns 0.67
-    against 0.45, 16 columns 0.42 against 0.61; 1.5 M edges 64 columns 0.25 against 0.22, 36 columns 0.18 against 0.21;
-    below that the grouping's dozen launches lose.  Unaligned widths above 32 would be copied to be gathered."""
-    return n_edges * c >= GROUP_VALUES and c >= GROUP_COLUMNS and (c <= 32 or c % 4 == 0)
+    The reductions cost per value, and more of it the fewer sources the edges share; the grouping costs per edge, and per
+    node for its offsets and rows.  Power-law sources of a 29 k node graph, reductions against grouping in us: 64 columns
+    1.1 M edges 179 / 156, 7 M 1086 / 554; 48 columns 1.5 M 186 / 184; 32 columns 2.2 M 177 / 188, 4.5 M 411 / 309; 30 columns
+    4.5 M 355 / 370, 7 M 621 / 535; 36 columns 4.5 M 448 / 393, 7 M 559 / 564; 24 columns 4.5 M 278 / 354.  With 100 k nodes
+    64 columns are level at 2 M edges, 32 and 48 at 4.5 M.  Evenly spread sources keep the reductions ahead throughout (64
+    columns, 2 M edges 136 / 226).  Widths between 36 and 44 gain nothing, unaligned ones above 32 would be copied to be
+    gathered."""
+    values = n_edges * c
+    if c >= 48 and c % 4 == 0:
+        return values >= GROUP_VALUES and n_edges >= 32 * n_nodes
+    return 28 <= c <= 32 and values >= 2 * GROUP_VALUES and n_edges >= 128 * n_nodes
 
 
 def _sum_by_source(msg, idx, n):
@@ -537,7 +544,7 @@ def _edge_to_vertex(msg, csc, flag):
             plan = SpmmPlan(off, E, chunk=DEFAULT_CHUNK)
             csc._jg_plan_ordered = plan
         return segment_aggregate(msg, ident[0], off, ident[1], n_out=n, plan=plan, ordered=True)
-    if flag == 0 and _group_by_source(E, c):
+    if flag == 0 and _group_by_source(E, n, c):
         try:
             return _sum_by_source(msg, idx, n)
         except torch.OutOfMemoryError:      # some 40 bytes an edge; the reductions below need none

@@ -466,3 +466,32 @@ def test_gatconv_takes_the_reference_constructor_call(cuda, oracle):
     assert np.abs(host(y1) - want).max() <= 1e-5 * np.abs(want).max() + 1e-6
     with pytest.raises(TypeError):
         nn.GATConv(64, 128)                                    # e_num is positional and required, as in the reference
+
+
+def test_sum_by_source_without_the_memory_to_group(cuda, monkeypatch):
+    """Where the grouping's arrays do not fit, the reductions do the sum."""
+    n, E, c = 40, 4099, 64
+    rng = np.random.default_rng(3)
+    idx, off = random_csc(rng, n, E)
+    csc, m = cuda.CSC(dev(idx), dev(off), None), rng.standard_normal((E, c)).astype(np.float32)
+    called = []
+
+    def no_memory(*args):
+        called.append(args)
+        raise torch.OutOfMemoryError("no room")
+
+    monkeypatch.setattr(cuda.ops, "_group_by_source", lambda *args: True)
+    monkeypatch.setattr(cuda.ops, "_sum_by_source", no_memory)
+    x = dev(np.zeros((n, c), np.float32)).requires_grad_(True)
+    cuda.ScatterToEdge(x, csc, "src").backward(dev(m))
+    want, mag = np.zeros((n, c)), np.zeros((n, c))
+    np.add.at(want, idx, m.astype(np.float64))
+    np.add.at(mag, idx, np.abs(m).astype(np.float64))
+    assert called and np.all(np.abs(host(x.grad) - want) <= np.bincount(idx, minlength=n).max() * 2.0**-24 * mag)
+
+
+@pytest.mark.parametrize("c", [32, 64])
+def test_grouping_looks_at_the_nodes(cuda, c):
+    """Enough values to group on a graph of few nodes; on one of many the offsets and rows of the groups cost more than the
+    reductions."""
+    assert cuda.ops._group_by_source(7_000_000, 30_000, c) and not cuda.ops._group_by_source(7_000_000, 4_000_000, c)
