@@ -6,6 +6,7 @@ calls a hand-written sm_100a kernel through the C ABI of ``libjgb200.so``; there
 is no CPU or eager fallback for any of them.
 """
 import ctypes
+import operator
 import os
 
 import torch
@@ -261,23 +262,18 @@ def aggregate_bias_act(x, csc, csr, bias=None, relu=False):
     return _AggregateBiasAct.apply(x, bias, csc, csr, bool(relu))
 
 
-def _entries(container):
-    """Indices, offsets and weights of a CSC or a CSR."""
-    if isinstance(container, CSC):
-        return container.row_indices, container.column_offset, container.edge_weight
-    return container.column_indices, container.row_offset, container.edge_weight
-
-
 class _Propagate(torch.autograd.Function):
     """``v <- keep * A v + restart * x`` from ``v = x``, ``hops`` times.  The result is a polynomial in A applied to
     x, so the gradient is the same recursion over the transposed structure, started from the output's gradient:
     nothing of the forward is kept."""
 
     @staticmethod
-    def forward(ctx, x, fwd, bwd, hops, restart):
-        ctx.fwd, ctx.bwd, ctx.hops, ctx.restart = fwd, bwd, hops, restart
-        idx, off, w = _entries(fwd)
-        plan = _plan_of(fwd, off, idx.numel())
+    def forward(ctx, x, csc, csr, hops, restart, transposed):
+        ctx.csc, ctx.csr, ctx.hops, ctx.restart, ctx.transposed = csc, csr, hops, restart, transposed
+        if transposed:
+            idx, off, w, plan = csr.column_indices, csr.row_offset, csr.edge_weight, _plan_of(csr, csr.row_offset, csr.column_indices.numel())
+        else:
+            idx, off, w, plan = csc.row_indices, csc.column_offset, csc.edge_weight, _plan_of(csc, csc.column_offset, csc.row_indices.numel())
         f = x.shape[1]
         h = _as_f32(x, "x")
         if f > 32 and f % 4:       # one padded copy for all hops
@@ -289,15 +285,17 @@ class _Propagate(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_output):
-        return _Propagate.apply(grad_output, ctx.bwd, ctx.fwd, ctx.hops, ctx.restart), None, None, None, None
+        g = _Propagate.apply(grad_output, ctx.csc, ctx.csr, ctx.hops, ctx.restart, not ctx.transposed)
+        return g, None, None, None, None, None
 
 
 def propagate(x, csc, csr, hops, restart):
     """``hops`` steps of ``v <- (1 - restart) * A v + restart * x`` starting at ``x``
     (nn/conv/appnp_conv.py:41-52), one kernel per hop in either direction."""
+    hops = operator.index(hops)          # a whole number: 2.5 hops are a mistake, not 2
     if hops <= 0:
         return x
-    return _Propagate.apply(x, csc, csr, int(hops), float(restart))
+    return _Propagate.apply(x, csc, csr, hops, float(restart), False)
 
 
 def _edge_index(edge_index):

@@ -382,3 +382,20 @@ def test_long_rows_on_either_kernel(cuda, f):
     far[:n_in] = x
     plan = cuda.ops.SpmmPlan(off, nnz, 256)
     assert torch.equal(cuda.ops.segment_aggregate(x, idx, off, w, plan=plan), cuda.ops.segment_aggregate(far, idx, off, w, plan=plan))
+
+
+def test_propagation_takes_what_it_took(cuda):
+    """Any object with the containers' fields is a container, and a number of hops is a whole number."""
+    from types import SimpleNamespace
+    from jittorgeometric_b200 import nn
+    n = 60
+    ei = torch.randint(0, n, (2, 300), device="cuda", dtype=torch.int32)
+    csc, csr = cuda.gcn_norm_csc_csr(ei, None, n)
+    x = torch.randn((n, 12), device="cuda", requires_grad=True)
+    y = nn.APPNP(3, 0.1)(x, csc, csr)
+    g, = torch.autograd.grad(y, x, torch.ones_like(y))
+    like = nn.APPNP(np.int64(3), 0.1)(x, SimpleNamespace(**vars(csc)), SimpleNamespace(**vars(csr)))
+    assert torch.equal(like, y) and torch.equal(torch.autograd.grad(like, x, torch.ones_like(y))[0], g)
+    with pytest.raises(TypeError):
+        nn.APPNP(2.5, 0.1)(x, csc, csr)
+    assert nn.APPNP(0, 0.1)(x, csc, csr) is x
