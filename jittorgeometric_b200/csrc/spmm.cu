@@ -25,6 +25,10 @@
 
 namespace jg {
 
+// The kernels walk entries by 32-bit positions in steps of 32, the streaming one two windows ahead of a ticket padded to
+// whole steps: beyond this a position would wrap before it reaches the end.
+constexpr int64_t kMaxEntries = INT32_MAX - 128;
+
 struct PlanHeader {
     int32_t n_hubs;
     int32_t n_items;
@@ -970,7 +974,7 @@ static int aggregate_impl(float* out, const float* x, const int32_t* idx, const 
     if (n_out == 0 || f == 0) return JG_OK;
     JG_CHECK_ARG(out && off, JG_EINVAL, "aggregate: null out/off");
     JG_CHECK_ARG(nnz == 0 || (x && idx && w), JG_EINVAL, "aggregate: null x/idx/w with nnz > 0");
-    JG_CHECK_ARG(n_out < INT32_MAX && n_in <= INT32_MAX && nnz <= INT32_MAX, JG_ESHAPE,
+    JG_CHECK_ARG(n_out < INT32_MAX && n_in <= INT32_MAX && nnz <= kMaxEntries, JG_ESHAPE,
                  "aggregate: sizes beyond int32 indexing");
     JG_CHECK_ARG(!plan || chunk > 0, JG_EINVAL, "aggregate: a plan needs the chunk it was built with");
     JG_CHECK_ARG(workspace, JG_EWORKSPACE, "aggregate: workspace is null");
@@ -1120,7 +1124,7 @@ int jg_aggregate_f32_static(float* out, const float* x, const int32_t* idx, cons
     if (n_out == 0 || f == 0) return JG_OK;
     JG_CHECK_ARG(out && off, JG_EINVAL, "aggregate_static: null out/off");
     JG_CHECK_ARG(nnz == 0 || (x && idx && w), JG_EINVAL, "aggregate_static: null x/idx/w with nnz > 0");
-    JG_CHECK_ARG(n_out < INT32_MAX && n_in <= INT32_MAX && nnz <= INT32_MAX, JG_ESHAPE,
+    JG_CHECK_ARG(n_out < INT32_MAX && n_in <= INT32_MAX && nnz <= kMaxEntries, JG_ESHAPE,
                  "aggregate_static: sizes beyond int32 indexing");
     // Piece length: 1024 entries, doubled until plan and partial rows fit the fixed array.
     int32_t chunk = 1024;

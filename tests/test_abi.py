@@ -44,6 +44,16 @@ def test_host_only_entry_points():
     assert L.jg_aggregate_workspace_bytes(10, 100, 8, 0) >= 8
 
 
+def test_aggregation_refuses_entry_counts_whose_positions_wrap():
+    """The largest counts are refused before anything is launched (the pointers here name nothing)."""
+    from jittorgeometric_b200 import _lib
+    L, p = _lib.lib(), 256
+    for nnz in (2**31 - 128, 2**31 - 1, 2**31):
+        assert L.jg_aggregate_f32(p, p, p, p, p, 10, 10, 8, nnz, None, 0, p, 1 << 20, None) == -2
+        assert L.jg_aggregate_f32_static(p, p, p, p, p, 10, 10, 8, nnz, None) == -2
+    assert L.jg_aggregate_f32(p, p, p, p, p, 10, 10, 8, 2**31 - 129, None, 0, None, 0, None) == -3      # only the workspace is missing
+
+
 def test_ops_refuse_cpu_tensors():
     import torch
     import jittorgeometric_b200 as jg
