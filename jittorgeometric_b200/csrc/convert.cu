@@ -11,7 +11,7 @@
 // Method: stable least-significant-digit radix sort, 8 bits per pass, ceil(bits(n)/8) passes,
 // carrying (key, other index, weight).  Each pass = per-tile digit histogram, one device-wide
 // exclusive scan of the [tile][digit] count matrix in digit-major order, and a stable scatter: ranks inside a tile come from
-// per-digit masks of the warp (votes) in element order, elements are staged in shared memory in digit order and
+// per-digit masks of the warp (votes, or matches on a list in runs) in element order, elements are staged in shared memory in digit order and
 // written out in coalesced runs.  The first pass reads the caller's COO directly (self-loop
 // removal and the appended loops are folded into it: removed entries are simply never counted),
 // the last pass writes the caller's output arrays.  Offsets are found from the sorted keys by
@@ -31,8 +31,8 @@ constexpr int kRadix = 256;
 // unit-weight entries, three passes, two formats: 14.9 against 15.9 ms), but a third array to carry spills
 // (30 M weighted entries: 3.1 against 2.6 ms), and a list of fewer than some 2 M entries would leave SMs
 // without a tile.
-constexpr int kMatchRuns = 8;      // runs of equal digits in 32 elements up to which a match mask beats the votes
 constexpr int kItemsFew = 8, kItemsMany = 16;
+constexpr int kMatchRuns = 8;      // runs of equal digits in 32 elements up to which a match mask beats the votes
 constexpr int64_t kManyEntries = (int64_t)1 << 21;
 static inline int sort_items(int64_t count, bool carry_w) { return !carry_w && count >= kManyEntries ? kItemsMany : kItemsFew; }
 static inline int64_t sort_tiles(int64_t count, int items) {
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kSortThreads, ITEMS == kItemsMany ? 3 : 4) sor
     for (int i = 0; i < kRadix / 32; i++) my_hist[i * 32 + lane] = 0;
     __syncwarp();
     const unsigned lt_mask = (1u << lane) - 1u;
-    // Ranking: lanes with the same digit find each other by a match mask, the first of them takes the group's
+    // Ranking: lanes with the same digit find each other (by match mask or votes), the first of them takes the group's
     // places with ONE shared-memory atomic and hands the start round.  The rounds' atomics are issued one behind
     // the other and their results picked up afterwards, so a round does not wait for the one before it (a
     // read, a warp barrier, a write and another warp barrier per round were a chain of eight shared-memory
@@ -1151,7 +1151,8 @@ int jg_gcn_norm_coo(const int32_t* edge_index, const float* w, int64_t n_edges, 
                  "gcn_norm_coo: workspace %zu < %zu", workspace_bytes, jg_gcn_norm_coo_workspace_bytes(n_edges, n_nodes));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     NormCooWs nw = carve_norm_coo(workspace, n_edges, n_nodes);
-    // degrees come from the destination-major order (sequential sums in list order); its arrays are scratch here
+    // degrees come from the destination-major order (sums in list order, by a fixed tree beyond kLongColumn entries); its
+    // arrays are scratch here
     int rc = jg_gcn_norm_compressed(edge_index, w, n_edges, n_nodes, fill, add_self_loops, 0, nw.tmp_idx, nw.tmp_off,
                                     nw.tmp_w, nullptr, nullptr, nullptr, out_count, nw.convert, nw.convert_bytes, stream);
     if (rc != JG_OK) return rc;

@@ -7,11 +7,11 @@
 // x^T * g (a reduction over the rows, the one operand layout the row-tiled kernel does not take) and
 // shapes the tensor-core kernel refuses.  With it no product of the path goes to a library.
 //
-// Operands are addressed by two strides each, A(i,l) = a[i*sa0 + l*sa1], B(l,j) = b[l*sb0 + j*sb1],
-// so x @ W, g @ W^T and x^T @ g are the same kernel.  64x64 output tile per CTA, 16-deep slices
-// through shared memory, 4x4 register block per thread, fp32 FMA.  A long reduction (x^T g over
-// millions of rows) is cut into slices across CTAs whose partial tiles are added in a fixed order by a
-// second kernel: no atomics, identical results run to run.
+// Operands are addressed by two strides each, A(i,l) = a[i*sa0 + l*sa1], B(l,j) = b[l*sb0 + j*sb1].
+// sgemm_kernel takes any strides (x @ W, g @ W^T): 64x64 output tile per CTA, 16-deep slices through shared
+// memory, 4x4 register block per thread, fp32 FMA.  sgemm_tn_kernel takes x^T @ g, both operands along their
+// rows.  A long reduction (millions of rows) is cut into slices across CTAs whose partial tiles are added in a
+// fixed order by a second kernel: no atomics, identical results run to run.
 #include "common.cuh"
 
 namespace jg {

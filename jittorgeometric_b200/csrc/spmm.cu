@@ -7,14 +7,16 @@
 //
 // Work decomposition.  A "work id" is either one piece (<= chunk entries) of a
 // hub row listed in the plan, or one ordinary row.  A persistent grid of warps
-// pulls ids eight at a time from a global ticket counter (hub pieces first, so
-// the longest items start earliest).  One warp owns one id: it reads 32 indices
-// and weights with one coalesced load each (the next tile, which may already
-// belong to the next row, is prefetched), stages them in shared memory as
-// (index, weight) pairs so that each entry costs one 64-bit broadcast load, and
-// gathers feature rows with 128-bit loads, a batch of rows in flight per lane.
-// Full batches run without predicates: the kernel is sensitive to instruction
-// issue as well as to memory latency (about 8-12 instructions per entry).
+// pulls tickets from a global counter, hub pieces first, so the longest items
+// start earliest; a ticket is one to eight ids, fewer the less work there is.
+// Who walks an id depends on the width:
+//   F <= 31            aggregate_narrow_kernel: 4 to 32 lanes a row, rows side by side
+//   F = 32, 36 .. 64   aggregate_stream_kernel, or row by row where that is faster
+//   F = 68 .. 512      aggregate_rows_kernel: a warp a row, 128-bit gathers
+//   any other          aggregate_any_kernel: scalar loads along the columns
+// Indices and weights are read 32 at a time, coalesced, ahead of their use; the
+// last three stage them in shared memory or hand them round with shuffles.  The
+// kernels are sensitive to instruction issue as well as to memory latency.
 // Memory-bound: per nonzero one 4 B index, one 4 B weight and one F*4 B row.
 //
 // Determinism.  Each output row is produced by exactly one warp (or, for a hub
@@ -346,12 +348,14 @@ __global__ void __launch_bounds__(kBlock, MINB) aggregate_rows_kernel(AggArgs a)
 // instantiation, so the plain kernel is untouched).  The width is a template parameter: with it in a register the
 // 40-column form was slower than the 64-column one.
 //
-// The segments of a ticket (rows, pieces of hub rows) are walked as ONE stream of entries, each segment padded to
-// whole steps: a window of 32 stream positions at a time is looked up by the lanes (position -> segment by a
+// The segments of a ticket (a piece of a hub row, or up to eight rows) are walked as ONE stream of entries, each segment
+// padded to whole steps: a window of 32 stream positions at a time is looked up by the lanes (position -> segment by a
 // search over the ticket's prefix lengths), staged in shared memory as (index, weight) pairs and marked where a
 // segment ends.  Batches of B steps are double-buffered in registers across row ends, so the gathers of the next
 // rows are in flight while a row is summed and stored; walked row by row, a row of a dozen entries cost two or
 // three exposed memory latencies.  The next ticket, and its segments' bounds, are fetched while this one is walked.
+// At 64 registers (four CTAs per SM) the plain and the combining form spill 32 bytes at 36 to 60 columns, the bias form 80,
+// both epilogues 80 at 64 columns, none at 32.
 template <int F, int B, int MINB, int EPI>
 __global__ void __launch_bounds__(kBlock, MINB) aggregate_stream_kernel(AggArgs a) {
     constexpr int G = F <= 32 ? 8 : 16;
@@ -370,7 +374,7 @@ __global__ void __launch_bounds__(kBlock, MINB) aggregate_stream_kernel(AggArgs 
     const int chunk = a.hdr ? a.hdr->chunk : 0x7fffffff;
     const int grab = a.grab;
     // a piece of a hub is a ticket of its own (with four of them in one warp a small graph's tail was longer than its
-    // work: 50 k rows, 1.3 M entries, 36 columns, both directions 0.20 ms against 0.12 of the row kernel on 16 lanes), rows come `grab` at a time
+    // work: 50 k rows, 1.3 M entries, 36 columns, both directions 0.20 ms, 0.12 row by row), rows come `grab` at a time
     const int64_t tickets = n_items + (a.n_out + grab - 1) / grab;
     auto first_id = [&](int64_t ticket) { return ticket < n_items ? ticket : n_items + (ticket - n_items) * grab; };
 
