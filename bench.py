@@ -113,20 +113,27 @@ def build_graph(device, scale=21, edge_factor=32):
     return jg.CSC(src.contiguous(), off, w.contiguous()), n
 
 
+def aggregation_code_sha256():
+    """Hash of the aggregation's source without its comments and spacing: what a capture of its counters belongs to."""
+    import hashlib
+    import re
+    text = open(os.path.join(ROOT, "jittorgeometric_b200", "csrc", "spmm.cu")).read()
+    code = re.sub(r"/\*.*?\*/|//[^\n]*", "", text, flags=re.S)
+    return hashlib.sha256("".join(code.split()).encode()).hexdigest()
+
+
 def measured_traffic(nnz, widths):
     """DRAM bytes (read + write) per aggregation launch at each width, from the committed table of ncu
     counters (``dram__bytes_read.sum + dram__bytes_write.sum``, one capture at full size).  The record is
-    used only for the workload it was taken on (same nonzero count) and only while the kernel source
+    used only for the workload it was taken on (same nonzero count) and only while the kernel code
     it was taken with is unchanged; otherwise there is no traffic figure (``None``)."""
-    import hashlib
     table = os.path.join(ROOT, "profiles", "dram_traffic.json")
-    src = os.path.join(ROOT, "jittorgeometric_b200", "csrc", "spmm.cu")
     try:
-        rec = json.load(open(table))["aggregate_rows_kernel"]["spmm_sweep"]
-        sha = hashlib.sha256(open(src, "rb").read()).hexdigest()
+        rec = json.load(open(table))["aggregation"]["spmm_sweep"]
+        sha = aggregation_code_sha256()
     except (OSError, KeyError, ValueError):
         return None
-    if rec.get("nnz") != nnz or rec.get("source_sha256") != sha:
+    if rec.get("nnz") != nnz or rec.get("code_sha256") != sha:
         return None
     out = {}
     for f in widths:
@@ -380,7 +387,7 @@ def run_single(args):
         "sweep": sweep,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak if achieved else None, "traffic": total_traffic, "peak_kind": peak_kind,
-                     "kernel": "aggregate_rows_kernel",
+                     "kernel": "aggregate_stream_kernel (32, 64 columns), aggregate_rows_kernel (128, 256)",
                      "model_gbs": total_bytes / kernel_ms / 1e6, "model_frac": total_bytes / kernel_ms / 1e6 / peak,
                      "min_gbs": total_min / kernel_ms / 1e6, "min_frac": total_min / kernel_ms / 1e6 / peak,
                      "note": "achieved / frac = DRAM bytes the four aggregation launches really move (ncu dram__bytes read + "

@@ -439,7 +439,8 @@ def run(args):
             "config": bench.workload_config(args.scale, args.edge_factor, n, nnz, world),
             "gflops": 2.0 * nnz * sum(widths) / (ms_step * 1e-3) / 1e9,
             "roofline": {"bound": "hbm", "achieved": None, "peak": peak, "unit": "GB/s", "frac": None, "traffic": None,
-                         "peak_kind": peak_kind, "kernel": "aggregate_rows_kernel",
+                         "peak_kind": peak_kind,
+                         "kernel": "aggregate_stream_kernel (32, 64 columns), aggregate_rows_kernel (128, 256)",
                          "model_gbs_per_gpu": total_bytes / world / ms_step / 1e6,
                          "model_frac": total_bytes / world / ms_step / 1e6 / peak,
                          "note": "no DRAM counter record for the partitioned run: frac is null; model_* = per-GPU bytes of the "
