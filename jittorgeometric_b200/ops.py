@@ -545,7 +545,7 @@ def _edge_to_vertex(msg, csc, flag):
     if flag == 0 and _group_by_source(E, n, c):
         try:
             return _sum_by_source(msg, idx, n)
-        except torch.OutOfMemoryError:      # some 40 bytes an edge; the reductions below need none
+        except torch.OutOfMemoryError:      # some 35 bytes an edge; the reductions below need none
             pass
     out = torch.empty((n, c), dtype=torch.float32, device=msg.device)
     check(lib().jg_edge_to_vertex_f32(ptr(out), ptr(msg), ptr(idx), ptr(off), n, E, c, flag, stream_for(msg)),
@@ -568,7 +568,8 @@ class _ScatterToEdgeFunc(torch.autograd.Function):
 
 def ScatterToEdge(x, csc, flow):
     """Node rows copied onto edges in CSC order: ``flow="src"`` takes each edge's source row,
-    anything else its destination row (ops/scatterToEdge.py:49-51)."""
+    anything else its destination row (ops/scatterToEdge.py:49-51).  The backward by source of a large edge tensor groups
+    the edges first (:func:`_group_by_source`) and takes some 35 bytes an edge of scratch for it, where there is room."""
     return _ScatterToEdgeFunc.apply(x, csc, flow)
 
 
