@@ -500,16 +500,15 @@ def _scatter_to_edge(x, csc, flag):
 def _group_by_source(n_edges, n_nodes, c):
     """Whether the sum per source groups the edges first (:func:`_sum_by_source`) or reduces into L2 in edge order.
     The reductions cost per value, and more of it the fewer sources the edges share; the grouping costs per edge, and per
-    node for its offsets and rows.  Power-law sources of a 29 k node graph, reductions against grouping in us: 64 columns
-    1.1 M edges 179 / 156, 7 M 1086 / 554; 48 columns 1.5 M 186 / 184; 32 columns 2.2 M 177 / 188, 4.5 M 411 / 309; 30 columns
-    4.5 M 355 / 370, 7 M 621 / 535; 36 columns 4.5 M 448 / 393, 7 M 559 / 564; 24 columns 4.5 M 278 / 354.  With 100 k nodes
-    64 columns are level at 2 M edges, 32 and 48 at 4.5 M.  Evenly spread sources keep the reductions ahead throughout (64
-    columns, 2 M edges 136 / 226).  Widths between 36 and 44 gain nothing, unaligned ones above 32 would be copied to be
-    gathered."""
-    values = n_edges * c
-    if c >= 48 and c % 4 == 0:
-        return values >= GROUP_VALUES and n_edges >= 32 * n_nodes
-    return 28 <= c <= 32 and values >= 2 * GROUP_VALUES and n_edges >= 128 * n_nodes
+    node for its offsets and rows.  Its sums are in a fixed order and five times closer to the exact ones, so it stays
+    where it is about level.  Power-law sources of a 29 k node graph, reductions against grouping in us: 64 columns
+    1.1 M edges 179 / 156, 7 M 1086 / 554; 48 columns 1.5 M 186 / 184; 36 columns 3 M 230 / 294, 4.5 M 448 / 393; 32 columns 2.2 M
+    177 / 188, 4.5 M 411 / 309; 30 columns 3 M 236 / 287, 7 M 621 / 535; 24 columns 3 M 185 / 273, 4.5 M 278 / 354.  With 100 k
+    nodes 64 columns are level at 2 M edges, 36 columns lose at 4.5 M (338 / 441).  Evenly spread sources keep the reductions
+    ahead throughout (64 columns, 2 M edges 136 / 226).  Unaligned widths above 32 would be copied to be gathered."""
+    if c < 28 or (c > 32 and c % 4):
+        return False
+    return n_edges * c >= GROUP_VALUES and n_edges >= (32 if c >= 48 else 128) * n_nodes
 
 
 def _sum_by_source(msg, idx, n):

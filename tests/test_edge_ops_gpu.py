@@ -495,3 +495,4 @@ def test_grouping_looks_at_the_nodes(cuda, c):
     """Enough values to group on a graph of few nodes; on one of many the offsets and rows of the groups cost more than the
     reductions."""
     assert cuda.ops._group_by_source(7_000_000, 30_000, c) and not cuda.ops._group_by_source(7_000_000, 4_000_000, c)
+    assert not cuda.ops._group_by_source(7_000_000, 30_000, 24) and not cuda.ops._group_by_source(7_000_000, 30_000, 49)
