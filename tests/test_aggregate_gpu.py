@@ -248,8 +248,8 @@ def test_fused_epilogue_autograd(cuda):
 @pytest.mark.parametrize("mode", ["plain", "epilogue", "accumulate", "combine"])
 @pytest.mark.parametrize("f", [5, 32, 36, 40, 44, 48, 64, 72, 130])
 def test_row_lengths_and_epilogues(cuda, oracle, f, mode):
-    """Rows of 0 to 34 entries in every order (runs of empty rows, segments that end on and beside step, batch and window
-    borders), rows one entry above and below the piece length, an infinite value in a row that no entry names.
+    """Rows of 0 to 34 entries in every order, runs of empty rows, rows one entry above and below the piece length, an
+    infinite value in a row that no entry names; so few rows are walked one by one (several a ticket: further down).
     A sum of k terms is off by at most k + 4 roundings (its epilogue's included) of the sum of magnitudes."""
     rng = np.random.default_rng(f)
     n_in = 500
